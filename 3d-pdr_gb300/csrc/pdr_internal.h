@@ -102,6 +102,11 @@ struct WarpTables {
   } sp;
 };
 
+// classes of the reactions that are not sums over the rays: what of
+// alpha (T/300)^beta exp(-gamma/T) they need; RC_GENERAL holds the other
+// kinds and parameters outside the fast path's ranges
+enum RateClass { RC_CONST = 0, RC_BETA, RC_GAMMA, RC_BOTH, RC_CRP, RC_CRPHOT, RC_GENERAL, RC_COUNT };
+
 // Device tables for the rate evaluator.
 struct RateTables {
   int nreac = 0;
@@ -116,7 +121,13 @@ struct RateTables {
   // grouped by kind (lanes of a warp then mostly take the same branch)
   int nray = 0, nother = 0;
   int *ray_reac = nullptr;    // [nray]
-  int *other_reac = nullptr;  // [nother]
+  int *other_reac = nullptr;  // [nother], grouped by RateClass
+  int class_off[RC_COUNT] = {}, class_n[RC_COUNT] = {};
+  float *beta_f = nullptr, *gamma_f = nullptr;
+  // the shielded reactions present, the C photo-rate's gamma, and whether the
+  // fast path takes the network's parameters
+  int has_h2 = 0, has_hd = 0, has_co = 0, has_ci = 0, fast_ok = 0;
+  double ci_gamma = 0.0;
 };
 
 struct HostNet {

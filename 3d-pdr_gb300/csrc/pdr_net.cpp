@@ -435,7 +435,42 @@ int build_device_tables(pdr_net *net) {
     for (int i = 0; i < h.nreac; i++) (ray_kind(h.rate_kind[i]) ? ray : other).push_back(i);
     auto by_kind = [&](int x, int y) { return h.rate_kind[x] < h.rate_kind[y]; };
     std::stable_sort(ray.begin(), ray.end(), by_kind);
+    // class of a reaction; |alpha|, |beta| and |gamma| within what keeps the fast
+    // path's exponents representable, and no grain reactant (whose rate may exceed 1)
+    auto rate_class = [&](int i) -> int {
+      const int k = h.rate_kind[i];
+      const double a = std::fabs(h.alpha[i]), b = h.beta[i], g = h.gamma[i];
+      if (k == RK_GRAIN) return std::isfinite(a) ? RC_CONST : RC_GENERAL;
+      if (!(a >= 1.0e-150 && a <= 1.0e100) || !(std::fabs(b) <= 100.0) || !(std::fabs(g) <= 1.0e7) || (flags[i] & 1))
+        return RC_GENERAL;
+      if (k == RK_CRP) return RC_CRP;
+      if (k == RK_CRPHOT) return RC_CRPHOT;
+      if (k != RK_THERMAL) return RC_GENERAL;
+      return b == 0.0 ? (g == 0.0 ? RC_CONST : RC_GAMMA) : (g == 0.0 ? RC_BETA : RC_BOTH);
+    };
     std::stable_sort(other.begin(), other.end(), by_kind);
+    std::stable_sort(other.begin(), other.end(), [&](int x, int y) { return rate_class(x) < rate_class(y); });
+    for (int i : other) net->rates.class_n[rate_class(i)]++;
+    for (int c = 1; c < RC_COUNT; c++)
+      net->rates.class_off[c] = net->rates.class_off[c - 1] + net->rates.class_n[c - 1];
+    bool fast = true, first_ci = true;
+    for (int i : ray) {
+      const int k = h.rate_kind[i];
+      net->rates.has_h2 |= k == RK_PHOTO_H2;
+      net->rates.has_hd |= k == RK_PHOTO_HD;
+      net->rates.has_co |= k == RK_PHOTO_CO;
+      net->rates.has_ci |= k == RK_PHOTO_CI;
+      if (k == RK_PHOTO_CI) {
+        if (!first_ci && h.gamma[i] != net->rates.ci_gamma) fast = false;   // one table of C photo-rates per ray
+        net->rates.ci_gamma = h.gamma[i];
+        first_ci = false;
+      }
+      if (!(h.gamma[i] >= 0.0 && h.gamma[i] <= 1.0e4) || !(std::fabs(h.alpha[i]) <= 1.0e100)) fast = false;
+    }
+    net->rates.fast_ok = fast ? 1 : 0;
+    std::vector<float> bf(h.beta.begin(), h.beta.end()), gf(h.gamma.begin(), h.gamma.end());
+    net->rates.beta_f = upload(net, bf, rc);
+    net->rates.gamma_f = upload(net, gf, rc);
     net->rates.nray = (int)ray.size();
     net->rates.nother = (int)other.size();
     net->rates.ray_reac = upload(net, ray, rc);
