@@ -13,8 +13,8 @@
 //   bool owns; bool leader();  void sync();
 //   double sum_all(double); float sum_all(float); double max_all(double);
 //   double rhs(double y_own);  bool setup(double y_own);  double solve(double b_own);
-//   and, for the mixed form, double solve32(double b_own, float gscale, float &x32)
-//   (the correction times gscale, in FP64 and in FP32);
+//   and, for the mixed form, float solve32(double b_own, float gscale)
+//   (the correction times gscale);
 // Norms are kept squared (the tests compare squares, no sqrt); the step-ratio
 // heuristics eta = 1/((bias*e)^(1/k) + 1e-6) are evaluated in FP32.
 #pragma once
@@ -87,11 +87,11 @@ __device__ __forceinline__ bool eq_u(double a, double b) {
 }
 
 // squared-norm form of eta = 1/((bias*e)^(1/k) + 1e-6) with e2 = e^2 (FP32)
-__device__ __forceinline__ double eta_of(float e2, float bias, int k) {
+__device__ __forceinline__ float eta_of(float e2, float bias, int k) {
   const float v = powf(bias * bias * e2, 0.5f / (float)k);
-  return (double)(1.0f / (v + (float)ADDON));
+  return 1.0f / (v + (float)ADDON);
 }
-__device__ __forceinline__ double eta_of(double e2, float bias, int k) { return eta_of((float)e2, bias, k); }
+__device__ __forceinline__ float eta_of(double e2, float bias, int k) { return eta_of((float)e2, bias, k); }
 
 // 1/x to double precision: FP32 seed and two Newton steps
 __device__ __forceinline__ double rcp_nr(double x) {
@@ -206,6 +206,7 @@ struct Core {
   ZT z;
   NT ewt;
   double acor, y, ftmp, tmp;
+  float acor32;   // mixed form: acor in FP32, set when the Newton iteration has converged
   // uniform integrator scalars
   double tn, h, hscale, hprime, eta, etamax, gamma, gammap, rl1;
   NT inv_gammap, gamrat, gscale, saved_tq5;
@@ -593,13 +594,18 @@ struct Core {
     self().sync();
   }
 
-  // store l[0..Q] of the FP32/FP64 recurrence as FP64 (only the used terms)
+  // store l[0..Q] of the FP32/FP64 recurrence (only the used terms): the mixed
+  // form reads l[1] in FP64 (l[0] is 1) and the rest in FP32, so that one
+  // conversion per step is left of six
   template <int Q>
   __device__ __forceinline__ void store_l(const NT *l) {
+    if constexpr (NORM32) {
+      ws->l[1] = (double)l[1];
 #pragma unroll
-    for (int j = 0; j <= Q; j++) {
-      ws->l[j] = (double)l[j];
-      ws->lf[j] = (float)l[j];
+      for (int j = 2; j <= Q; j++) ws->lf[j] = (float)l[j];
+    } else {
+#pragma unroll
+      for (int j = 0; j <= Q; j++) ws->l[j] = (double)l[j];
     }
   }
 
@@ -617,10 +623,13 @@ struct Core {
       if constexpr (NORM32) h_nt = ws->tauf[1];
       else h_nt = h;
       if (self().leader()) {
+        if constexpr (NORM32) {
+          ws->l[1] = wu->ul[q][1];
 #pragma unroll
-        for (int j = 0; j <= QMAX; j++) {
-          ws->l[j] = wu->ul[q][j];
-          ws->lf[j] = wu->ulf[q][j];
+          for (int j = 2; j <= QMAX; j++) ws->lf[j] = wu->ulf[q][j];
+        } else {
+#pragma unroll
+          for (int j = 0; j <= QMAX; j++) ws->l[j] = wu->ul[q][j];
         }
         ws->rl1 = wu->url1[q];
         tq[2] = utqn(q, 2);
@@ -681,19 +690,23 @@ struct Core {
         if (!self().setup(y)) return fail;
         call_setup = false;
       }
-      acor = 0.0;
       NT delp2 = 0;
       int mcor = 0;
       bool conv = false;
       const double rz1 = rl1 * z[1];   // fixed during the iteration
+      // the first iteration starts from acor = 0: its residual, correction and
+      // norm need no sum with acor and no second conversion of it (a third of
+      // the Newton update's FP64 instructions; one iteration converges in 4 of
+      // 5 steps)
       for (;;) {
-        tmp = gamma * ftmp - (rz1 + acor);
+        tmp = fma(gamma, ftmp, -(mcor > 0 ? rz1 + acor : rz1));
         NT del2;
+        float t32 = 0.0f;
         if constexpr (NORM32) {
           // the FP32 solve returns the correction already scaled by gscale,
           // and its FP32 value feeds the norm
-          float t32;
-          tmp = self().solve32(tmp, gscale, t32);
+          t32 = self().solve32(tmp, gscale);
+          tmp = (double)t32;
           del2 = wrms2_32(t32);
         } else {
           tmp = self().solve(tmp);
@@ -701,11 +714,15 @@ struct Core {
           del2 = wrms2(tmp);
         }
         nni++;
-        acor += tmp;
-        y = z[0] + acor;
+        acor = (mcor > 0) ? acor + tmp : tmp;
         if (mcor > 0) crate2 = fmax(NT(CRDOWN * CRDOWN) * crate2, del2 / delp2);
         if (del2 * fmin(NT(1), crate2) <= tq4sq) {
-          acnrm2 = (mcor == 0) ? del2 : wrms2(acor);
+          if constexpr (NORM32) {
+            acor32 = (mcor == 0) ? t32 : (float)acor;
+            acnrm2 = (mcor == 0) ? del2 : wrms2_32(self().owns ? acor32 : 0.0f);
+          } else {
+            acnrm2 = (mcor == 0) ? del2 : wrms2(acor);
+          }
           jcur = 0;
           conv = true;
           break;
@@ -713,6 +730,7 @@ struct Core {
         mcor++;
         if (mcor == MAXCOR || (mcor >= 2 && del2 > NT(RDIV * RDIV) * delp2)) break;
         delp2 = del2;
+        y = z[0] + acor;
         ftmp = self().rhs(y);
       }
       if (conv) return 0;
@@ -722,9 +740,11 @@ struct Core {
     return fail;
   }
 
-  __device__ __forceinline__ void set_eta() {
-    if (lt_u(eta, THRESH)) { eta = 1.0; hprime = h; }
-    else { eta = fmin(eta, etamax); hprime = h * eta; }
+  // the step ratio is an FP32 value: it is compared and limited as one, and
+  // only a ratio that changes the step becomes FP64
+  __device__ __forceinline__ void set_eta(float r) {
+    if (r < (float)THRESH) { eta = 1.0; hprime = h; }
+    else { eta = (double)fminf(r, (float)etamax); hprime = h * eta; }
   }
 
   // one internal step: 0 ok, CVODE flag (<0), or FELL_BACK
@@ -769,8 +789,7 @@ struct Core {
       etamax = 1.0;
       const int L = q + 1;
       if (nef <= MXNEF1) {
-        eta = eta_of(dsm2, (float)BIAS2, L);
-        eta = fmax(ETAMIN, eta);
+        eta = fmax(ETAMIN, (double)eta_of(dsm2, (float)BIAS2, L));
         if (nef >= SMALL_NEF) eta = fmin(eta, ETAMXF);
         rescale();
         continue;
@@ -809,13 +828,11 @@ struct Core {
       }
     }
     self().sync();
-    // mixed form: the FP32 value of the correction for the FP32 columns, the
-    // order-raise save and the order heuristics
-    float acor32 = 0.0f;
+    // mixed form: acor32, the FP32 value of the correction, serves the FP32
+    // columns, the order-raise save and the order heuristics
     if constexpr (NORM32) {
-      z[0] = fma(ws->l[0], acor, z[0]);
+      z[0] = z[0] + acor;   // l[0] = 1
       z[1] = fma(ws->l[1], acor, z[1]);
-      acor32 = (float)acor;
       if constexpr (ZSHARED) {
 #pragma unroll 1
         for (int j = 2; j <= q; j++) z.setf(j, fmaf(ws->lf[j], acor32, z.getf(j)));
@@ -845,14 +862,13 @@ struct Core {
       eta = 1.0;
     } else {
       const int L = q + 1;
-      const double etaq = eta_of(dsm2, (float)BIAS2, L);
+      const float etaq = eta_of(dsm2, (float)BIAS2, L);
       if (qwait != 0) {
-        eta = etaq;
         qprime = q;
-        set_eta();
+        set_eta(etaq);
       } else {
         qwait = 2;
-        double etaqm1 = 0.0, etaqp1 = 0.0;
+        float etaqm1 = 0.0f, etaqp1 = 0.0f;
         if (q > 1) {
           const NT tq1 = tqn()[1];
           if constexpr (NORM32) {
@@ -882,17 +898,18 @@ struct Core {
             etaqp1 = eta_of(wrms2(acor - (double)cquot * z[QMAX]) * (tq3 * tq3), (float)BIAS3, L + 1);
         }
         // ties keep the current order, then prefer the lower one
-        const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
-        if (etam < THRESH) { eta = 1.0; qprime = q; }
-        else if (etam == etaq) { eta = etaq; qprime = q; }
-        else if (etam == etaqm1) { eta = etaqm1; qprime = q - 1; }
+        const float etam = fmaxf(etaqm1, fmaxf(etaq, etaqp1));
+        float r = 1.0f;
+        if (etam < (float)THRESH) { qprime = q; }
+        else if (etam == etaq) { r = etaq; qprime = q; }
+        else if (etam == etaqm1) { r = etaqm1; qprime = q - 1; }
         else {
-          eta = etaqp1;
+          r = etaqp1;
           qprime = q + 1;
           if constexpr (NORM32) z.setf(QMAX, acor32);
           else z[QMAX] = acor;
         }
-        set_eta();
+        set_eta(r);
       }
     }
     etamax = (nst <= SMALL_NST) ? ETAMX2 : ETAMX3;

@@ -807,14 +807,12 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
   }
 
   // mixed form: the residual converted once and scaled in FP32 (the scaling
-  // of the FP32 matrix); the correction comes back times ssc*gscale, in FP32
-  // for the norm and in FP64 for the state
-  __device__ __forceinline__ double solve32(double b, float gs, float &x32) {
+  // of the FP32 matrix); the correction comes back times ssc*gscale
+  __device__ __forceinline__ float solve32(double b, float gs) {
     MT xv;
     if constexpr (SP) xv = sparse_solve(owns ? (float)b * wsc32 : 0.0f);
     else xv = lin_solve(owns ? (float)b * wsc32 : 0.0f);
-    x32 = owns ? xv * (ssc32 * gs) : 0.0f;
-    return (double)x32;
+    return owns ? xv * (ssc32 * gs) : 0.0f;
   }
 
   // the triangular solves with the factors in place: v is this thread's

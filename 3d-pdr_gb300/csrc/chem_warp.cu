@@ -441,12 +441,10 @@ struct WarpCell : Core<WarpCell<NSP, MIXED, ZSH>, ZSH, MIXED> {
   }
 
   // mixed form: the residual is converted once and scaled in FP32 (the
-  // scaling of the FP32 matrix), the correction comes back times ssc*gscale,
-  // in FP32 for the norm and in FP64 for the state
-  __device__ __forceinline__ double solve32(double b, float gs, float &x32) {
+  // scaling of the FP32 matrix), the correction comes back times ssc*gscale
+  __device__ __forceinline__ float solve32(double b, float gs) {
     const float xv = lu_solve_rows<NSP, float>(jrow, LDJ, lane, mystep, invd, (float)b * wsc32, perm);
-    x32 = owns ? xv * (ssc32 * gs) : 0.0f;
-    return (double)x32;
+    return owns ? xv * (ssc32 * gs) : 0.0f;
   }
 
   // calculate_abundances.c:132-317 for one cell
