@@ -54,8 +54,8 @@ struct CoefShared {
   float lf[QMAX + 1];   // l in FP32 (the mixed form's FP32 Nordsieck columns)
 };
 
-// coefficients of a uniform step history (xi_j = j), per order 1..5: the
-// same for every integrator, so one copy serves a whole block
+// coefficients of a uniform step history (xi_j = j), per order 1..5, evaluated
+// by the compiler (the recurrence of Core::coeffs with h = tau_j = 1)
 struct CoefUniform {
   double ul[QMAX + 1][QMAX + 1];
   double url1[QMAX + 1];
@@ -63,6 +63,49 @@ struct CoefUniform {
   float utqf[QMAX + 1][6];
   float ulf[QMAX + 1][QMAX + 1];
 };
+constexpr CoefUniform uniform_coefficients() {
+  CoefUniform u{};
+  for (int q = 1; q <= QMAX; q++) {
+    double l[QMAX + 1] = {1.0, 1.0}, tq[6] = {};
+    double a0 = -1.0, a0hat = -1.0, xi_inv = 1.0, xistar_inv = 1.0, hsum = 1.0;
+    if (q > 1) {
+      for (int j = 2; j < q; j++) {
+        hsum += 1.0;
+        xi_inv = 1.0 / hsum;
+        a0 -= 1.0 / j;
+        for (int i = j; i >= 1; i--) l[i] += l[i - 1] * xi_inv;
+      }
+      a0 -= 1.0 / q;
+      xistar_inv = -l[1] - a0;
+      hsum += 1.0;
+      xi_inv = 1.0 / hsum;
+      a0hat = -l[1] - xi_inv;
+      for (int i = q; i >= 1; i--) l[i] += l[i - 1] * xistar_inv;
+    }
+    auto mag = [](double x) { return x < 0.0 ? -x : x; };
+    const double A1 = 1.0 - a0hat + a0, A2 = 1.0 + q * A1;
+    tq[2] = mag(A1 / (a0 * A2));
+    tq[5] = mag(A2 * xistar_inv / (l[q] * xi_inv));
+    const double C = xistar_inv / l[q], A3 = a0 + 1.0 / q, A4 = a0hat + xi_inv;
+    tq[1] = q > 1 ? mag(C * (1.0 - A4 + A3) / A3) : 1.0;
+    hsum += 1.0;
+    xi_inv = 1.0 / hsum;
+    const double A5 = a0 - 1.0 / (q + 1), A6 = a0hat - xi_inv;
+    tq[3] = mag(((1.0 - A6 + A5) / A2) / (xi_inv * (q + 2) * A5));
+    tq[4] = NLSCOEF / tq[2];
+    for (int j = 0; j <= QMAX; j++) {
+      u.ul[q][j] = l[j];
+      u.ulf[q][j] = (float)l[j];
+    }
+    u.url1[q] = 1.0 / l[1];
+    for (int j = 1; j <= 5; j++) {
+      u.utqd[q][j] = tq[j];
+      u.utqf[q][j] = (float)tq[j];
+    }
+  }
+  return u;
+}
+static __constant__ CoefUniform c_uniform = uniform_coefficients();
 
 // Comparisons of uniform FP64 scalars in integer arithmetic: for operands
 // whose sign bits are clear, the bit patterns order like the values, and NaN
@@ -91,7 +134,6 @@ __device__ __forceinline__ float eta_of(float e2, float bias, int k) {
   const float v = powf(bias * bias * e2, 0.5f / (float)k);
   return 1.0f / (v + (float)ADDON);
 }
-__device__ __forceinline__ float eta_of(double e2, float bias, int k) { return eta_of((float)e2, bias, k); }
 
 // 1/x to double precision: FP32 seed and two Newton steps
 __device__ __forceinline__ double rcp_nr(double x) {
@@ -199,7 +241,6 @@ struct Core {
   using NT = typename std::conditional<NORM32, float, double>::type;
   __device__ __forceinline__ D &self() { return *static_cast<D *>(this); }
   CoefShared *ws = nullptr;
-  CoefUniform *wu = nullptr;   // the uniform-history table (may be shared by several integrators)
   // Nordsieck row of this thread's species, weight, correction, work values
   using ZT = typename std::conditional<NORM32, typename std::conditional<ZSHARED, ZSharedM, ZRowM>::type,
                                        typename std::conditional<ZSHARED, ZShared, ZRow>::type>::type;
@@ -223,8 +264,8 @@ struct Core {
     else return ws->tqd;
   }
   __device__ __forceinline__ NT utqn(int qq, int j) const {
-    if constexpr (NORM32) return wu->utqf[qq][j];
-    else return wu->utqd[qq][j];
+    if constexpr (NORM32) return c_uniform.utqf[qq][j];
+    else return c_uniform.utqd[qq][j];
   }
   __device__ __forceinline__ const NT *taun() const {
     if constexpr (NORM32) return ws->tauf;
@@ -296,40 +337,50 @@ struct Core {
       }
     }
   }
-  // the same with a run-time order, rolled (rows in shared memory)
+  // the same with a run-time order (rows in shared memory): the row is taken
+  // into registers once, with zeros for the columns above q (the triangle
+  // leaves them and what they are added to unchanged), and its columns 2..q
+  // are stored once
   template <int SIGN>
-  __device__ __forceinline__ void pascal_m_rolled() {
+  __device__ __forceinline__ void pascal_m_q() {
     if (q == 1) {
       z[0] = (SIGN > 0) ? z[0] + z[1] : z[0] - z[1];
       return;
     }
+    float f[QMAX + 1];
+#pragma unroll
+    for (int j = 2; j <= QMAX; j++) f[j] = (j <= q) ? z.getf(j) : 0.0f;
+    const double z0 = z[0], z1 = z[1];
     float s0 = 0.0f, s1 = 0.0f;
     if (SIGN > 0) {
-#pragma unroll 1
-      for (int j = 2; j <= q; j++) { const float f = z.getf(j); s0 += f; s1 = fmaf((float)j, f, s1); }
+#pragma unroll
+      for (int j = 2; j <= QMAX; j++) { s0 += f[j]; s1 = fmaf((float)j, f[j], s1); }
     }
-#pragma unroll 1
-    for (int k = 1; k <= q; k++)
-#pragma unroll 1
-      for (int j = q; j >= (k > 3 ? k : 3); j--)
-        z.setf(j - 1, (SIGN > 0) ? z.getf(j - 1) + z.getf(j) : z.getf(j - 1) - z.getf(j));
+#pragma unroll
+    for (int k = 1; k <= QMAX; k++)
+#pragma unroll
+      for (int j = QMAX; j >= (k > 3 ? k : 3); j--) f[j - 1] = (SIGN > 0) ? f[j - 1] + f[j] : f[j - 1] - f[j];
     if (SIGN < 0) {
-#pragma unroll 1
-      for (int j = 2; j <= q; j++) { const float f = z.getf(j); s0 += f; s1 = fmaf((float)j, f, s1); }
+#pragma unroll
+      for (int j = 2; j <= QMAX; j++) { s0 += f[j]; s1 = fmaf((float)j, f[j], s1); }
     }
+#pragma unroll
+    for (int j = 2; j < QMAX; j++)
+      if (j < q) z.setf(j, f[j]);   // column q itself does not change
     if (SIGN > 0) {
-      z[0] = z[0] + (z[1] + (double)s0);
-      z[1] = z[1] + (double)s1;
+      z[0] = z0 + (z1 + (double)s0);
+      z[1] = z1 + (double)s1;
     } else {
-      z[1] = z[1] - (double)s1;
-      z[0] = z[0] - (z[1] + (double)s0);
+      const double w = z1 - (double)s1;
+      z[1] = w;
+      z[0] = z0 - (w + (double)s0);
     }
   }
   template <int SIGN>
   __device__ __forceinline__ void pascal_q() {
     if constexpr (NORM32) {
       if constexpr (ZSHARED) {
-        pascal_m_rolled<SIGN>();
+        pascal_m_q<SIGN>();
       } else {
         switch (q) {
           case 1: pascal_m<1, SIGN>(); break;
@@ -522,28 +573,43 @@ struct Core {
   // Newton correction and the error-test thresholds, so FP32 perturbs the
   // solution by ~1e-7 of the correction (itself of the size of the local
   // error), and the ~10 divisions here cost FP32 instead of FP64 issue slots
+  //
+  // The divisions, a dozen one after the other, are made side by side instead:
+  // lane m divides h by the sum of h and the last m steps, the five quotients
+  // of the second round and the three of the last have a lane each.  (An FP64
+  // division is 7 FP64 instructions, an inlined FP32 one a dozen; the warp pays
+  // for one whatever its active lanes.)  Every lane of the warp calls it with
+  // the same arguments and gets the same results; rl1 = 1/l[1].
   template <class T>
-  __device__ __forceinline__ static void coeffs(int q, bool order_change_due, T h, const T *tau, T *l, T *tq) {
+  __device__ __forceinline__ static void coeffs(int q, bool order_change_due, T h, const T *tau, T *l, T *tq, T &rl1) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    T hsum = h;
+#pragma unroll
+    for (int i = 1; i <= QMAX; i++)
+      if (i <= lane && i <= q) hsum += tau[i];
+    const T ratio = h / hsum;   // xi_inv after lane steps of history
+    auto inverse = [](int n) -> T {   // 1/n, n = 1..6
+      return n == 1 ? T(1) : n == 2 ? T(1) / T(2) : n == 3 ? T(1) / T(3) : n == 4 ? T(1) / T(4) : n == 5 ? T(1) / T(5) : T(1) / T(6);
+    };
 #pragma unroll
     for (int j = 0; j <= QMAX; j++) l[j] = T(0);
     l[0] = l[1] = T(1);
-    T a0 = T(-1), a0hat = T(-1), xi_inv = T(1), xistar_inv = T(1), hsum = h;
+    T a0 = T(-1), a0hat = T(-1), xi_inv = T(1), xistar_inv = T(1);
     if (q > 1) {
 #pragma unroll
       for (int j = 2; j < QMAX; j++) {
+        const T x = __shfl_sync(FULL, ratio, j - 1);
         if (j < q) {
-          hsum += tau[j - 1];
-          xi_inv = h / hsum;
           a0 -= T(1) / T(j);
 #pragma unroll
           for (int i = QMAX; i >= 1; i--)
-            if (i <= j) l[i] += l[i - 1] * xi_inv;
+            if (i <= j) l[i] += l[i - 1] * x;
         }
       }
-      a0 -= T(1) / T(q);
+      a0 -= inverse(q);
       xistar_inv = -l[1] - a0;
-      hsum += tau[q - 1];
-      xi_inv = h / hsum;
+      xi_inv = __shfl_sync(FULL, ratio, q - 1);
       a0hat = -l[1] - xi_inv;
 #pragma unroll
       for (int i = QMAX; i >= 1; i--)
@@ -553,45 +619,28 @@ struct Core {
 #pragma unroll
     for (int j = 0; j <= QMAX; j++) if (j == q) lq = l[j];
     const T A1 = T(1) - a0hat + a0, A2 = T(1) + T(q) * A1;
-    tq[2] = fabs(A1 / (a0 * A2));
-    tq[5] = fabs(A2 * xistar_inv / (lq * xi_inv));
+    const T xi2 = __shfl_sync(FULL, ratio, q);
+    const T A5 = a0 - inverse(q + 1), A6 = a0hat - xi2;
+    T num = T(1), den = l[1];
+    if (lane == 0) { num = A1; den = a0 * A2; }
+    else if (lane == 1) { num = A2 * xistar_inv; den = lq * xi_inv; }
+    else if (lane == 2) { num = xistar_inv; den = lq; }
+    else if (lane == 3) { num = T(1) - A6 + A5; den = A2; }
+    T quot = num / den;
+    tq[2] = fabs(__shfl_sync(FULL, quot, 0));
+    tq[5] = fabs(__shfl_sync(FULL, quot, 1));
+    const T C = __shfl_sync(FULL, quot, 2), A3 = a0 + inverse(q), A4 = a0hat + xi_inv;
+    const T q3 = __shfl_sync(FULL, quot, 3);
+    rl1 = __shfl_sync(FULL, quot, 4);
+    if (lane == 0) { num = C * (T(1) - A4 + A3); den = A3; }
+    else if (lane == 1) { num = q3; den = xi2 * T(q + 2) * A5; }
+    else { num = T(NLSCOEF); den = tq[2]; }
+    quot = num / den;
     if (order_change_due) {
-      if (q > 1) {
-        const T C = xistar_inv / lq, A3 = a0 + T(1) / T(q), A4 = a0hat + xi_inv;
-        tq[1] = fabs(C * (T(1) - A4 + A3) / A3);
-      } else {
-        tq[1] = T(1);
-      }
-      hsum += tau[q];
-      xi_inv = h / hsum;
-      const T A5 = a0 - T(1) / T(q + 1), A6 = a0hat - xi_inv;
-      tq[3] = fabs(((T(1) - A6 + A5) / A2) / (xi_inv * T(q + 2) * A5));
+      tq[1] = (q > 1) ? fabs(__shfl_sync(FULL, quot, 0)) : T(1);
+      tq[3] = fabs(__shfl_sync(FULL, quot, 1));
     }
-    tq[4] = T(NLSCOEF) / tq[2];
-  }
-
-  // the table of uniform-history coefficients (h = tau_j = 1)
-  __device__ __forceinline__ void build_uniform_table() {
-    double one[QMAX + 2];
-#pragma unroll
-    for (int j = 0; j < QMAX + 2; j++) one[j] = 1.0;
-    for (int qq = 1; qq <= QMAX; qq++) {
-      double l[QMAX + 1], tq[6];
-      coeffs<double>(qq, true, 1.0, one, l, tq);
-      self().sync();
-      if (self().leader()) {
-        for (int j = 0; j <= QMAX; j++) {
-          wu->ul[qq][j] = l[j];
-          wu->ulf[qq][j] = (float)l[j];
-        }
-        wu->url1[qq] = 1.0 / l[1];
-        for (int j = 1; j <= 5; j++) {
-          wu->utqd[qq][j] = tq[j];
-          wu->utqf[qq][j] = (float)tq[j];
-        }
-      }
-    }
-    self().sync();
+    tq[4] = __shfl_sync(FULL, quot, 2);
   }
 
   // store l[0..Q] of the FP32/FP64 recurrence (only the used terms): the mixed
@@ -624,14 +673,14 @@ struct Core {
       else h_nt = h;
       if (self().leader()) {
         if constexpr (NORM32) {
-          ws->l[1] = wu->ul[q][1];
+          ws->l[1] = c_uniform.ul[q][1];
 #pragma unroll
-          for (int j = 2; j <= QMAX; j++) ws->lf[j] = wu->ulf[q][j];
+          for (int j = 2; j <= QMAX; j++) ws->lf[j] = c_uniform.ulf[q][j];
         } else {
 #pragma unroll
-          for (int j = 0; j <= QMAX; j++) ws->l[j] = wu->ul[q][j];
+          for (int j = 0; j <= QMAX; j++) ws->l[j] = c_uniform.ul[q][j];
         }
-        ws->rl1 = wu->url1[q];
+        ws->rl1 = c_uniform.url1[q];
         tq[2] = utqn(q, 2);
         tq[4] = utqn(q, 4);
         tq[5] = utqn(q, 5);
@@ -639,10 +688,10 @@ struct Core {
       }
     } else {
       h_nt = (NT)h;
-      NT l[QMAX + 1], tqv[6];
+      NT l[QMAX + 1], tqv[6], r;
       tqv[1] = tq[1];
       tqv[3] = tq[3];
-      coeffs<NT>(q, qwait == 1, h_nt, taun(), l, tqv);
+      coeffs<NT>(q, qwait == 1, h_nt, taun(), l, tqv, r);
       if (self().leader()) {
         switch (q) {
           case 1: store_l<1>(l); break;
@@ -651,7 +700,7 @@ struct Core {
           case 4: store_l<4>(l); break;
           default: store_l<5>(l); break;
         }
-        ws->rl1 = (double)(NT(1) / l[1]);
+        ws->rl1 = (double)r;
         tq[1] = tqv[1]; tq[2] = tqv[2]; tq[3] = tqv[3]; tq[4] = tqv[4]; tq[5] = tqv[5];
       }
     }
@@ -683,61 +732,65 @@ struct Core {
     const NT tq4 = tqn()[4];
     const NT tq4sq = tq4 * tq4;
     const int fail = fallback_on_fail ? 2 : 1;
-    for (int attempt = 0; attempt < 2; attempt++) {
-      y = z[0];
+    // one loop over the corrector iterations of up to two attempts, so that the
+    // right-hand side, the setup and the solve have one call site each: they are
+    // inlined, and the warps of an SM, at different phases, share its
+    // instruction cache
+    y = z[0];
+    bool second = false;
+    int mcor = 0;
+    NT delp2 = 0;
+    const double rz1 = __dmul_rn(rl1, z[1]);   // fixed during the iteration (rounded, not fused into the sum)
+    for (;;) {
       ftmp = self().rhs(y);
       if (call_setup) {
         if (!self().setup(y)) return fail;
         call_setup = false;
       }
-      NT delp2 = 0;
-      int mcor = 0;
-      bool conv = false;
-      const double rz1 = rl1 * z[1];   // fixed during the iteration
       // the first iteration starts from acor = 0: its residual, correction and
       // norm need no sum with acor and no second conversion of it (a third of
       // the Newton update's FP64 instructions; one iteration converges in 4 of
       // 5 steps)
-      for (;;) {
-        tmp = fma(gamma, ftmp, -(mcor > 0 ? rz1 + acor : rz1));
-        NT del2;
-        float t32 = 0.0f;
-        if constexpr (NORM32) {
-          // the FP32 solve returns the correction already scaled by gscale,
-          // and its FP32 value feeds the norm
-          t32 = self().solve32(tmp, gscale);
-          tmp = (double)t32;
-          del2 = wrms2_32(t32);
-        } else {
-          tmp = self().solve(tmp);
-          if (gscale != NT(1)) tmp *= (double)gscale;
-          del2 = wrms2(tmp);
-        }
-        nni++;
-        acor = (mcor > 0) ? acor + tmp : tmp;
-        if (mcor > 0) crate2 = fmax(NT(CRDOWN * CRDOWN) * crate2, del2 / delp2);
-        if (del2 * fmin(NT(1), crate2) <= tq4sq) {
-          if constexpr (NORM32) {
-            acor32 = (mcor == 0) ? t32 : (float)acor;
-            acnrm2 = (mcor == 0) ? del2 : wrms2_32(self().owns ? acor32 : 0.0f);
-          } else {
-            acnrm2 = (mcor == 0) ? del2 : wrms2(acor);
-          }
-          jcur = 0;
-          conv = true;
-          break;
-        }
-        mcor++;
-        if (mcor == MAXCOR || (mcor >= 2 && del2 > NT(RDIV * RDIV) * delp2)) break;
-        delp2 = del2;
-        y = z[0] + acor;
-        ftmp = self().rhs(y);
+      tmp = fma(gamma, ftmp, -(mcor > 0 ? rz1 + acor : rz1));
+      NT del2;
+      float t32 = 0.0f;
+      if constexpr (NORM32) {
+        // the FP32 solve returns the correction already scaled by gscale,
+        // and its FP32 value feeds the norm
+        t32 = self().solve32(tmp, gscale);
+        tmp = (double)t32;
+        del2 = wrms2_32(t32);
+      } else {
+        tmp = self().solve(tmp);
+        if (gscale != NT(1)) tmp *= (double)gscale;
+        del2 = wrms2(tmp);
       }
-      if (conv) return 0;
-      if (!jcur) { call_setup = true; continue; }
-      return fail;
+      nni++;
+      acor = (mcor > 0) ? acor + tmp : tmp;
+      if (mcor > 0) crate2 = fmax(NT(CRDOWN * CRDOWN) * crate2, del2 / delp2);
+      if (del2 * fmin(NT(1), crate2) <= tq4sq) {
+        if constexpr (NORM32) {
+          acor32 = (mcor == 0) ? t32 : (float)acor;
+          acnrm2 = (mcor == 0) ? del2 : wrms2_32(self().owns ? acor32 : 0.0f);
+        } else {
+          acnrm2 = (mcor == 0) ? del2 : wrms2(acor);
+        }
+        jcur = 0;
+        return 0;
+      }
+      mcor++;
+      if (mcor == MAXCOR || (mcor >= 2 && del2 > NT(RDIV * RDIV) * delp2)) {
+        // not converging: once more with a fresh matrix, unless it is fresh
+        if (jcur || second) return fail;
+        second = true;
+        call_setup = true;
+        mcor = 0;
+        y = z[0];
+        continue;
+      }
+      delp2 = del2;
+      y = z[0] + acor;
     }
-    return fail;
   }
 
   // the step ratio is an FP32 value: it is compared and limited as one, and
@@ -789,7 +842,7 @@ struct Core {
       etamax = 1.0;
       const int L = q + 1;
       if (nef <= MXNEF1) {
-        eta = fmax(ETAMIN, (double)eta_of(dsm2, (float)BIAS2, L));
+        eta = fmax(ETAMIN, (double)eta_of((float)dsm2, (float)BIAS2, L));
         if (nef >= SMALL_NEF) eta = fmin(eta, ETAMXF);
         rescale();
         continue;
@@ -833,14 +886,13 @@ struct Core {
     if constexpr (NORM32) {
       z[0] = z[0] + acor;   // l[0] = 1
       z[1] = fma(ws->l[1], acor, z[1]);
-      if constexpr (ZSHARED) {
-#pragma unroll 1
-        for (int j = 2; j <= q; j++) z.setf(j, fmaf(ws->lf[j], acor32, z.getf(j)));
-      } else {
+      float f[QMAX + 1];
 #pragma unroll
-        for (int j = 2; j <= QMAX; j++)
-          if (j <= q) z.setf(j, fmaf(ws->lf[j], acor32, z.getf(j)));
-      }
+      for (int j = 2; j <= QMAX; j++)
+        if (j <= q) f[j] = fmaf(ws->lf[j], acor32, z.getf(j));
+#pragma unroll
+      for (int j = 2; j <= QMAX; j++)
+        if (j <= q) z.setf(j, f[j]);
     } else if constexpr (ZSHARED) {
 #pragma unroll 1
       for (int j = 0; j <= q; j++) z[j] = fma(ws->l[j], acor, z[j]);
@@ -862,41 +914,56 @@ struct Core {
       eta = 1.0;
     } else {
       const int L = q + 1;
-      const float etaq = eta_of(dsm2, (float)BIAS2, L);
-      if (qwait != 0) {
-        qprime = q;
-        set_eta(etaq);
-      } else {
-        qwait = 2;
-        float etaqm1 = 0.0f, etaqp1 = 0.0f;
-        if (q > 1) {
+      // the step ratios of this order and, when a change of order is due, of the
+      // orders below and above: one evaluation, a lane for each
+      const int lane = threadIdx.x & 31;
+      float e2 = (float)dsm2, bias = (float)BIAS2;
+      int root = L;
+      bool lower = false, raise = false;
+      if (qwait == 0) {
+        lower = q > 1;
+        raise = q != QMAX && saved_tq5 != NT(0);
+        if (lower) {
           const NT tq1 = tqn()[1];
+          NT w;
           if constexpr (NORM32) {
             float zq = 0.0f;
 #pragma unroll
             for (int j = 2; j <= QMAX; j++) if (j == q) zq = z.getf(j);
-            etaqm1 = eta_of(wrms2_32(zq) * (tq1 * tq1), (float)BIAS1, q);
+            w = wrms2_32(zq);
           } else {
             double zq = 0.0;
 #pragma unroll
             for (int j = 0; j <= QMAX; j++) if (j == q) zq = z[j];
-            etaqm1 = eta_of(wrms2(zq) * (tq1 * tq1), (float)BIAS1, q);
+            w = wrms2(zq);
           }
+          if (lane == 1) { e2 = (float)(w * (tq1 * tq1)); bias = (float)BIAS1; root = q; }
         }
-        if (q != QMAX && saved_tq5 != NT(0)) {
+        if (raise) {
           // step-ratio factor of the order-raise estimate (heuristic, FP32)
           float ratio;
           if constexpr (NORM32) ratio = h_nt / ws->tauf[2];
           else ratio = (float)h / (float)ws->tau[2];
           float rp = ratio;
+#pragma unroll 1
           for (int k = 1; k < L; k++) rp *= ratio;
           const float cquot = ((float)tqn()[5] / (float)saved_tq5) * rp;
           const NT tq3 = tqn()[3];
-          if constexpr (NORM32)
-            etaqp1 = eta_of(wrms2_32(fmaf(-cquot, z.getf(QMAX), acor32)) * (tq3 * tq3), (float)BIAS3, L + 1);
-          else
-            etaqp1 = eta_of(wrms2(acor - (double)cquot * z[QMAX]) * (tq3 * tq3), (float)BIAS3, L + 1);
+          NT w;
+          if constexpr (NORM32) w = wrms2_32(fmaf(-cquot, z.getf(QMAX), acor32));
+          else w = wrms2(acor - (double)cquot * z[QMAX]);
+          if (lane == 2) { e2 = (float)(w * (tq3 * tq3)); bias = (float)BIAS3; root = L + 1; }
         }
+      }
+      const float etas = eta_of(e2, bias, root);
+      const float etaq = __shfl_sync(0xffffffffu, etas, 0);
+      if (qwait != 0) {
+        qprime = q;
+        set_eta(etaq);
+      } else {
+        qwait = 2;
+        const float e1 = __shfl_sync(0xffffffffu, etas, 1), e3 = __shfl_sync(0xffffffffu, etas, 2);
+        const float etaqm1 = lower ? e1 : 0.0f, etaqp1 = raise ? e3 : 0.0f;
         // ties keep the current order, then prefer the lower one
         const float etam = fmaxf(etaqm1, fmaxf(etaq, etaqp1));
         float r = 1.0f;
@@ -928,6 +995,7 @@ struct Core {
     if (hub < hlb) return hg;
     bool ok = false;
     double hnew = hg;
+#pragma unroll 1
     for (int it = 1; it <= 4; it++) {
       tmp = self().rhs(z[0] + hg * z[1]);
       const double yddnrm = sqrt(wrms2((tmp - z[1]) / hg));

@@ -78,7 +78,7 @@ struct CtaArgs {
 
 // byte offsets of the block's shared arrays (host and device agree)
 struct CtaLayout {
-  size_t scr, xs, part, red, sig, perm, cols, bsv, ys, upan, ws, wu, mat, dinv, yv, rfs, idx, wv, total;
+  size_t scr, xs, part, red, sig, perm, cols, bsv, ys, upan, ws, mat, dinv, yv, rfs, idx, wv, total;
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -106,7 +106,6 @@ __host__ __device__ inline CtaLayout cta_layout(const WarpTables &T, int ld, siz
   // LU panel; also the assembly's boundary slots (at most 2G - 2)
   L.upan = o; o += al16(mt * (size_t)(PB * n > 2 * G ? PB * n : 2 * G));
   L.ws = o; o += al16(sizeof(CoefShared));
-  L.wu = o; o += al16(sizeof(CoefUniform));
   L.mat = o;
   if (sp) {
     o += al16(mt * (size_t)T.sp.total);
@@ -946,7 +945,6 @@ __global__ void __launch_bounds__(256, SP ? 2 : 1) chem_cta_kernel(const __grid_
   c.ys = reinterpret_cast<MT *>(smem_raw + L.ys);
   c.upan = reinterpret_cast<MT *>(smem_raw + L.upan);
   c.ws = reinterpret_cast<CoefShared *>(smem_raw + L.ws);
-  c.wu = reinterpret_cast<CoefUniform *>(smem_raw + L.wu);
   c.mat = mat_smem ? reinterpret_cast<MT *>(smem_raw + L.mat)
                    : reinterpret_cast<MT *>(A.mat_global) + (size_t)blockIdx.x * (A.n + 2) * A.ld;
   c.dmat = c.mat;
@@ -961,7 +959,6 @@ __global__ void __launch_bounds__(256, SP ? 2 : 1) chem_cta_kernel(const __grid_
     c.wv = reinterpret_cast<MT *>(smem_raw + L.wv);
     c.stage_sparse(smem_raw + L.idx);
   }
-  c.build_uniform_table();
   if (total_ptr) total_cells = *total_ptr;
   __shared__ int next_idx;
   for (int k = 0;; k++) {
@@ -1016,7 +1013,6 @@ __global__ void __launch_bounds__(256, 1) eval_cta_kernel(const __grid_constant_
   c.ys = reinterpret_cast<double *>(smem_raw + L.ys);
   c.upan = reinterpret_cast<double *>(smem_raw + L.upan);
   c.ws = reinterpret_cast<CoefShared *>(smem_raw + L.ws);
-  c.wu = reinterpret_cast<CoefUniform *>(smem_raw + L.wu);
   c.mat = mat_smem ? reinterpret_cast<double *>(smem_raw + L.mat)
                    : reinterpret_cast<double *>(A.mat_global) + (size_t)blockIdx.x * (n + 2) * A.ld;
   c.dmat = c.mat;

@@ -176,6 +176,13 @@ __device__ __forceinline__ double rcp_seed(double b) {
   bits += (long long)__float2int_rn(y1 * 2251799813685248.0f) << 2;             // 2^51
   return __longlong_as_double(bits | (long long)((unsigned long long)(h & 0x80000000u) << 32));
 }
+// 1/b, rounded (2 FP64 instructions where the operand and result are normal)
+__device__ __forceinline__ double rcp_rn(double b) {
+  const unsigned e = ((unsigned)hi32(b) >> 20) & 0x7ff;
+  if (e - 2u >= 2042u) return __drcp_rn(b);   // zero, denormal, infinite, NaN, or a denormal result
+  const double y = rcp_seed(b);
+  return fma(y, fma(-b, y, 1.0), y);
+}
 // a/b for normal operands and result
 __device__ __forceinline__ double div_fast(double a, double b) {
   const double y = rcp_seed(b);

@@ -48,6 +48,22 @@ struct WarpTables {
   int2 *rhs_t = nullptr;      // [rhs_len][lanes] (kn index | (partial slot written after the term + 1) << 16,
                               //  operand | sign of nu << 31)
   int2 *pairs = nullptr;      // [npairs] slots (a, b) of each reactant pair
+  // The warp integrator's term tables in one packed block of `wtab_words` ints,
+  // which a block copies to shared memory (offsets in ints):
+  //   rt   [rhs_len4][32]  kn index << 3 | operand << 18 | sign of nu << 31 | 1 on the last term of a partial sum
+  //   h    [hlen4][32]     which * nreac + reaction | kind << 14 | nu << 16 (signed, 5 bits) | target << 21,
+  //                       target = row * 33 + column of the Newton matrix, or the slot
+  //                       (both padded to whole groups of four with terms that add a zero)
+  //   pk   [pk_len][32]   the pair products in the order rhs() forms them, slot a | slot b << 8 | operand << 16
+  //                       (operand 0: none): rounds 0..4 share their instruction with the levels of the x_e
+  //                       sum (lanes 16 >> round and up are free), the others follow, with every pair of the
+  //                       electron among them
+  //   pl   [1+plist_len][32] bytes: first partial slot of each lane, then the partial slots of each species
+  //   rab  [nreac] 16-bit: slot a | slot b << 8
+  //   bnd  [nbnd]         target | first slot << 11 | last slot + 1 << 19 of the runs across chunks
+  int pk_len = 0, nslots = 0, rhs_len4 = 0, hlen4 = 0;
+  int wt_rt = 0, wt_h = 0, wt_pk = 0, wt_pl = 0, wt_rab = 0, wt_bnd = 0, wtab_words = 0;
+  int *wtab = nullptr;
   int *kext_ptr = nullptr;    // [nkext+1] extra rate constant e = sum over kext_rn[kext_ptr[e]..kext_ptr[e+1])
   int2 *kext_rn = nullptr;    //   of nu * kn_r, (reaction r, nu) in reaction order
   int *plist = nullptr;       // [plist_len][lanes] partial slots of species `lane`

@@ -707,8 +707,83 @@ int build_device_tables(pdr_net *net) {
       if (neq + 1 > 255) return PDR_E_NET;
       if (G > kWarp ? slot > 8 * neq : slot > w.nparts) return PDR_E_NET;
       w.nbnd = (int)bt.size();
+      w.nslots = slot;
+    }
+    // the warp integrator's packed tables (pdr_internal.h); a network beyond
+    // their fields (8,191 rate constants) is left to the block integrator
+    std::vector<int> wt;
+    if (G == kWarp) {
+      if (nkn >= 8192 || w.nparts >= 127 || w.nop >= 1024 || neq * (kWarp + 1) + kWarp >= 2048 || w.nslots >= 255)
+        return PDR_E_NET;
+      std::vector<int> free_pairs, el_pairs, pk;
+      for (int p = 0; p < (int)pairs.size(); p++)
+        (pairs[p].x == neq || pairs[p].y == neq ? el_pairs : free_pairs).push_back(p);
+      auto word = [&](int p) { return pairs[p].x | (pairs[p].y << 8) | ((neq + 2 + p) << 16); };
+      pk.assign(5 * kWarp, 0);
+      size_t at = 0;
+      for (int k = 0; k < 5; k++)
+        for (int l = 16 >> k; l < kWarp && at < free_pairs.size(); l++) pk[k * kWarp + l] = word(free_pairs[at++]);
+      std::vector<int> rest(free_pairs.begin() + at, free_pairs.end());
+      rest.insert(rest.end(), el_pairs.begin(), el_pairs.end());
+      for (size_t i = 0; i < rest.size(); i++) {
+        if (i % kWarp == 0) pk.resize(pk.size() + kWarp, 0);
+        pk[(5 + i / kWarp) * kWarp + i % kWarp] = word(rest[i]);
+      }
+      w.pk_len = (int)pk.size() / kWarp;
+      w.wt_rt = 0;
+      w.rhs_len4 = (w.rhs_len + 3) & ~3;
+      w.hlen4 = (w.hlen + 3) & ~3;
+      // a lane's partial slots follow one another, so a term only marks the end of a sum
+      std::vector<unsigned char> plb(kWarp, 0);
+      for (int l = 0, next = 0; l < kWarp; l++) {
+        plb[l] = (unsigned char)next;
+        for (int t = 0; t < w.rhs_len; t++) {
+          const int fl = (int)((unsigned)rt[t * kWarp + l].x >> 16);
+          if (fl && fl - 1 != next++) return PDR_E_NET;
+        }
+      }
+      for (int t = 0; t < w.rhs_len4; t++)
+        for (int l = 0; l < kWarp; l++) {
+          const int2 e = t < w.rhs_len ? rt[t * kWarp + l] : make_int2(nkn, ONE);
+          wt.push_back((int)((((unsigned)e.x & 0xffffu) << 3) | (((unsigned)e.y & 0x7ffu) << 18) |
+                             ((unsigned)e.y & 0x80000000u) | ((unsigned)e.x >> 16 ? 1u : 0u)));
+        }
+      w.wt_h = (int)wt.size();
+      for (const int2 &t : hxy) {
+        const unsigned r = (unsigned)t.x & 0xffffu, which = ((unsigned)t.x >> 16) & 1u, kind = ((unsigned)t.x >> 17) & 3u;
+        const int nu = t.x >> 19;
+        if (nu < -16 || nu > 15) return PDR_E_NET;
+        const unsigned row = (unsigned)t.y & 0xffu, col = ((unsigned)t.y >> 8) & 0xffu, slot = (unsigned)t.y >> 16;
+        const unsigned target = kind == 2 ? slot : row * (kWarp + 1) + col;
+        wt.push_back((int)((which * (unsigned)h.nreac + r) | (kind << 14) | (((unsigned)nu & 31u) << 16) | (target << 21)));
+      }
+      wt.resize(w.wt_h + (size_t)w.hlen4 * kWarp, 0);
+      w.wt_pk = (int)wt.size();
+      wt.insert(wt.end(), pk.begin(), pk.end());
+      auto bytes = [&](const std::vector<unsigned char> &v) {
+        const int off = (int)wt.size();
+        wt.resize(wt.size() + (v.size() + 3) / 4, 0);
+        std::memcpy(wt.data() + off, v.data(), v.size());
+        return off;
+      };
+      plb.insert(plb.end(), pl.begin(), pl.end());
+      std::vector<unsigned char> rb;
+      for (const int2 &ab : rab) {
+        rb.push_back((unsigned char)ab.x);
+        rb.push_back((unsigned char)ab.y);
+      }
+      w.wt_pl = bytes(plb);
+      w.wt_rab = bytes(rb);
+      w.wt_bnd = (int)wt.size();
+      for (size_t i = 0; i < bt.size(); i++) {
+        const unsigned row = (unsigned)bt[i] & 0xffu, col = ((unsigned)bt[i] >> 8) & 0xffu;
+        wt.push_back((int)((row * (kWarp + 1) + col) | (((unsigned)bs[i] & 0xffu) << 11) | ((((unsigned)bs[i] >> 16) & 0xffu) << 19)));
+      }
+      while (wt.size() % 4) wt.push_back(0);
+      w.wtab_words = (int)wt.size();
     }
     int rc2 = 0;
+    if (!wt.empty()) w.wtab = upload(net, wt, rc2);
     w.rab = upload(net, rab, rc2);
     w.nh_mask = upload(net, nhm, rc2);
     w.rhs_t = upload(net, rt, rc2);
