@@ -152,11 +152,19 @@ int build_coolant_tables(pdr_coolant *c) {
     for (int k = 0; k < h.ntemp; k++)
       for (int e = 0; e < nn; e++) col.push_back(h.col[((size_t)p * nn + e) * h.ntemp + k]);
   }
+  std::vector<double> dcol(col.size(), 0.0);
+  for (int q = 0; q < t.npart; q++)
+    for (int k = 0; k + 1 < h.ntemp; k++)
+      for (int e = 0; e < nn; e++) {
+        const size_t at = ((size_t)q * h.ntemp + k) * nn + e;
+        dcol[at] = col[at + nn] - col[at];
+      }
   std::vector<int> lop(nn, -1);
   for (int l = 0; l < h.nlin; l++) lop[h.line_up[l] * n + h.line_lo[l]] = l;
   int rc = 0;
   t.temps = up(c, temps, rc);
   t.col = up(c, col, rc);
+  t.dcol = up(c, dcol, rc);
   t.A = up(c, h.A, rc);
   t.B = up(c, h.B, rc);
   t.freq = up(c, h.freq, rc);
@@ -194,6 +202,28 @@ int build_coolant_tables(pdr_coolant *c) {
       cmb[k] = tmp2[k] * (1.0 / (std::exp(HP * f / KB / 2.7) - 1.0));
       emis[k] = (double)0.01f * ((double)1.3f * f / 3.0e11);
     }
+    std::vector<double> hk(rp.size()), ahf(rp.size()), ab(rp.size() * 4), g(rp.size() * 2);
+    std::vector<int> ij(rp.size()), po(nn, 0);
+    for (size_t k = 0; k < rp.size(); k++) {
+      const int i = rp[k] / n, j = rp[k] % n, et = j * n + i;
+      hk[k] = HP * h.freq[rp[k]] / KB;
+      ahf[k] = h.A[rp[k]] * HP * h.freq[rp[k]];
+      ab[4 * k] = h.A[rp[k]];
+      ab[4 * k + 1] = h.B[rp[k]];
+      ab[4 * k + 2] = h.A[et];
+      ab[4 * k + 3] = h.B[et];
+      g[2 * k] = h.weights[i];
+      g[2 * k + 1] = h.weights[j];
+      ij[k] = i | (j << 8) | ((lop[rp[k]] + 1) << 16);
+      po[rp[k]] = (int)k + 1;
+      po[et] = -((int)k + 1);
+    }
+    t.pair_hk = up(c, hk, rc);
+    t.pair_ahf = up(c, ahf, rc);
+    t.pair_ab = up(c, ab, rc);
+    t.pair_g = up(c, g, rc);
+    t.pair_ij = up(c, ij, rc);
+    t.pair_of = up(c, po, rc);
     t.rad_pairs = up(c, rp, rc);
     t.pair_tmp2 = up(c, tmp2, rc);
     t.pair_cmb = up(c, cmb, rc);

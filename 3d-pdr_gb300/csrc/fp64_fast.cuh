@@ -189,6 +189,12 @@ __device__ __forceinline__ double div_fast(double a, double b) {
   const double q = a * y;
   return fma(fma(-q, b, a), y, q);
 }
+// a/b: div_fast where both and the quotient are normal with room, else the division
+__device__ __forceinline__ double div_any(double a, double b) {
+  const unsigned ea = ((unsigned)hi32(a) >> 20) & 0x7ff, eb = ((unsigned)hi32(b) >> 20) & 0x7ff;
+  if (ea - 64u > 1918u || eb - 64u > 1918u || ea - eb + 959u > 1918u) return a / b;
+  return div_fast(a, b);
+}
 // 1/sqrt(x), x positive normal within FP32's range
 __device__ __forceinline__ double rsqrt_fast(double x) {
   float y0;

@@ -175,6 +175,7 @@ struct CoolantTables {
   int part[7] = {0, 0, 0, 0, 0, 0, 0};   // LAMDA partner ids (0-based) with rates, ascending
   double *temps = nullptr;     // [npart][ntemp]
   double *col = nullptr;       // [npart][ntemp][nlev*nlev]
+  double *dcol = nullptr;      // [npart][ntemp][nlev*nlev] col[k+1] - col[k] (0 for the last)
   double *A = nullptr, *B = nullptr, *freq = nullptr, *weights = nullptr;
   double *energies = nullptr;  // [nlev] level energies, erg
   int *line_of_pair = nullptr; // [nlev*nlev] radiative line of (i,j), i>j, else -1
@@ -183,6 +184,12 @@ struct CoolantTables {
   double *pair_tmp2 = nullptr; // [nrad] 2 h nu^3 / c^2
   double *pair_cmb = nullptr;  // [nrad] tmp2 / (exp(h nu / k 2.7 K) - 1)
   double *pair_emis = nullptr; // [nrad] 0.01 (1.3 nu / 3e11), the dust emissivity factor
+  double *pair_hk = nullptr;   // [nrad] h nu / k
+  double *pair_ahf = nullptr;  // [nrad] A h nu
+  double *pair_ab = nullptr;   // [nrad][4] A_ij, B_ij, A_ji, B_ji
+  double *pair_g = nullptr;    // [nrad][2] statistical weights g_i, g_j
+  int *pair_ij = nullptr;      // [nrad] i | j << 8 | (radiative line + 1) << 16
+  int *pair_of = nullptr;      // [nlev*nlev] radiative pair + 1 of an entry, negative for (j, i), 0: none
   int *line_up = nullptr, *line_lo = nullptr;   // [nlin] levels of each radiative line
   double *line_frac1 = nullptr;                 // [nlin] A c^3 / (8 pi nu^3)
 };
