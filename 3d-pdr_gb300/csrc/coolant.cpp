@@ -169,6 +169,11 @@ int build_coolant_tables(pdr_coolant *c) {
   t.B = up(c, h.B, rc);
   t.freq = up(c, h.freq, rc);
   t.weights = up(c, h.weights, rc);
+  {
+    std::vector<double> rw(n);
+    for (int i = 0; i < n; i++) rw[i] = 1.0 / h.weights[i];
+    t.rweights = up(c, rw, rc);
+  }
   t.energies = up(c, h.energies, rc);
   t.line_of_pair = up(c, lop, rc);
   std::vector<int> rp;

@@ -195,6 +195,16 @@ __device__ __forceinline__ double div_any(double a, double b) {
   if (ea - 64u > 1918u || eb - 64u > 1918u || ea - eb + 959u > 1918u) return a / b;
   return div_fast(a, b);
 }
+// sqrt(x), rounded: six FP64 instructions where x is within FP32's normal range
+__device__ __forceinline__ double sqrt_rn(double x) {
+  if ((unsigned)hi32(x) - 0x38200000u > 0x0f000000u) return __dsqrt_rn(x);   // zero, negative, tiny, huge, NaN
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d2f(x)));
+  const double y = f2d(y0), g = x * y, h = scale2(y, -1);
+  const double r = fma(-g, h, 0.5);              // (1 - x y^2)/2
+  const double g1 = fma(g, r, g), h1 = fma(h, r, h);
+  return fma(fma(-g1, g1, x), h1, g1);
+}
 // 1/sqrt(x), x positive normal within FP32's range
 __device__ __forceinline__ double rsqrt_fast(double x) {
   float y0;

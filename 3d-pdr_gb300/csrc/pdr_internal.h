@@ -176,7 +176,7 @@ struct CoolantTables {
   double *temps = nullptr;     // [npart][ntemp]
   double *col = nullptr;       // [npart][ntemp][nlev*nlev]
   double *dcol = nullptr;      // [npart][ntemp][nlev*nlev] col[k+1] - col[k] (0 for the last)
-  double *A = nullptr, *B = nullptr, *freq = nullptr, *weights = nullptr;
+  double *A = nullptr, *B = nullptr, *freq = nullptr, *weights = nullptr, *rweights = nullptr;   // rweights: 1/weights
   double *energies = nullptr;  // [nlev] level energies, erg
   int *line_of_pair = nullptr; // [nlev*nlev] radiative line of (i,j), i>j, else -1
   int nrad = 0;

@@ -16,6 +16,7 @@
 // whose point lists are adjacent in memory.
 #include <algorithm>
 
+#include "fp64_fast.cuh"
 #include "pdr_internal.h"
 
 namespace pdr {
@@ -23,13 +24,15 @@ namespace {
 
 constexpr double PC = 3.08568025e+18;   // parsec in cm (healpix_types.F90:98)
 constexpr int SG = 8;                     // species per thread in the columns kernel
+constexpr int UV_THREADS = 192;           // 16 cells of 12 rays
+constexpr int TAU_THREADS = 256, TAU_STEPS = 8;
 
 // |x_i - x_{i-1}| as the reference writes it: sqrt((dx^2 + dy^2) + dz^2)
 __device__ __forceinline__ double step_length(const double *xyz, long long p) {
   const double dx = __dsub_rn(xyz[3 * (p - 1)], xyz[3 * p]);
   const double dy = __dsub_rn(xyz[3 * (p - 1) + 1], xyz[3 * p + 1]);
   const double dz = __dsub_rn(xyz[3 * (p - 1) + 2], xyz[3 * p + 2]);
-  return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+  return fp64::sqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
 }
 
 struct UvArgs {
@@ -44,39 +47,61 @@ struct UvArgs {
   double *colden, *AV, *rad, *uv;
 };
 
-__global__ void uvfield_kernel(const __grid_constant__ UvArgs A) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < A.ncell; c += gridDim.x * blockDim.x) {
-    double uv = 0.0;
-    for (int j = 0; j < A.nrays; j++) {
-      const size_t cj = (size_t)c * A.nrays + j;
-      const int ne = A.epray[cj];
-      double col = 0.0;
-      const long long pstart = A.offset[cj];
-      if (ne > 0 && (pstart < 0 || pstart + ne >= A.npoint)) col = nan("");
-      else if (ne > 0) {
-        const long long p0 = pstart;
-        const int g0 = A.gp[p0];
-        double rho_prev = (g0 >= 0 && g0 < A.ngrid) ? A.rho[g0] : nan("");
-        for (int i = 1; i <= ne; i++) {
-          const long long p = p0 + i;
-          const int gi = A.gp[p];
-          const double rho_i = (gi >= 0 && gi < A.ngrid) ? A.rho[gi] : nan("");
-          const double step = step_length(A.xyz, p);
-          col = __dadd_rn(col, __dmul_rn(__dmul_rn(__dadd_rn(rho_prev, rho_i) * 0.5, step), PC));
-          rho_prev = rho_i;
-        }
-      }
-      const double av = __dmul_rn(col, A.av_fac);
-      double rad = 0.0;
-      if (A.field == 0) rad = A.g_iso;
-      else if (j == A.uni_ray) rad = A.g_uni;
-      A.colden[cj] = col;
-      A.AV[cj] = av;
-      A.rad[cj] = rad;
-      uv = __dadd_rn(uv, __dmul_rn(rad, exp(__dmul_rn(-av, A.uv_fac))));
-      if (uv < 1.0e-50) uv = 0.0;
+// total-H column of one ray (NaN where an index leaves the grid)
+__device__ __forceinline__ double ray_column(const UvArgs &A, size_t cj) {
+  const int ne = A.epray[cj];
+  const long long p0 = A.offset[cj];
+  if (ne > 0 && (p0 < 0 || p0 + ne >= A.npoint)) return nan("");
+  double col = 0.0;
+  if (ne > 0) {
+    const int g0 = A.gp[p0];
+    double rho_prev = (g0 >= 0 && g0 < A.ngrid) ? A.rho[g0] : nan("");
+    for (int i = 1; i <= ne; i++) {
+      const long long p = p0 + i;
+      const int gi = A.gp[p];
+      const double rho_i = (gi >= 0 && gi < A.ngrid) ? A.rho[gi] : nan("");
+      const double step = step_length(A.xyz, p);
+      col = __dadd_rn(col, __dmul_rn(__dmul_rn(__dadd_rn(rho_prev, rho_i) * 0.5, step), PC));
+      rho_prev = rho_i;
     }
-    A.uv[c] = uv;
+  }
+  return col;
+}
+
+// A thread per (cell, ray) -- one per cell left a lattice of 29^3 cells with
+// one block per SM -- then the field of each cell is added in ray order, with
+// the reference's clamp after every ray, by one of its threads.  More rays
+// than a block has threads are taken in rounds.
+__global__ void __launch_bounds__(UV_THREADS) uvfield_kernel(const __grid_constant__ UvArgs A) {
+  __shared__ double term[UV_THREADS];
+  const int per = max(1, UV_THREADS / A.nrays);   // cells per block
+  for (long long base = (long long)blockIdx.x * per; base < A.ncell; base += (long long)gridDim.x * per) {
+    const int nb = (int)min((long long)per, A.ncell - base);
+    double uv = 0.0;
+    for (int j0 = 0; j0 < A.nrays; j0 += UV_THREADS) {
+      const int nj = min(A.nrays - j0, UV_THREADS);   // all rays, unless they are taken in rounds
+      const int c = threadIdx.x / nj, j = j0 + threadIdx.x - c * nj;
+      if (c < nb) {
+        const size_t cj = (size_t)(base + c) * A.nrays + j;
+        const double col = ray_column(A, cj);
+        const double av = __dmul_rn(col, A.av_fac);
+        double rad = 0.0;
+        if (A.field == 0) rad = A.g_iso;
+        else if (j == A.uni_ray) rad = A.g_uni;
+        A.colden[cj] = col;
+        A.AV[cj] = av;
+        A.rad[cj] = rad;
+        term[threadIdx.x] = __dmul_rn(rad, exp(__dmul_rn(-av, A.uv_fac)));
+      }
+      __syncthreads();
+      if (threadIdx.x < nb)
+        for (int q = 0; q < nj; q++) {
+          uv = __dadd_rn(uv, term[threadIdx.x * nj + q]);
+          if (uv < 1.0e-50) uv = 0.0;
+        }
+      __syncthreads();
+    }
+    if (threadIdx.x < nb) A.uv[base + threadIdx.x] = uv;
   }
 }
 
@@ -120,13 +145,14 @@ __global__ void columns_kernel(const __grid_constant__ ColArgs A) {
         int gi = A.gp[p];
         if (gi < 0 || gi >= A.ngrid) { bad = true; break; }
         const double ri = A.rho[gi];
-        const double sp = __dmul_rn(step_length(A.xyz, p), PC);
+        // half the step (exact), so that the trapezoid's factor costs nothing per species
+        const double sp = __dmul_rn(__dmul_rn(step_length(A.xyz, p), PC), 0.5);
         const double *xa = A.ab + (size_t)gprev * A.nspec, *xb = A.ab + (size_t)gi * A.nspec;
 #pragma unroll
         for (int u = 0; u < SG; u++)
           if (u < ns) {
             const double mid = __dadd_rn(__dmul_rn(rprev, xa[k[u]]), __dmul_rn(ri, xb[k[u]]));
-            acc[u] = __dadd_rn(acc[u], __dmul_rn(sp, mid) * 0.5);
+            acc[u] = __dadd_rn(acc[u], __dmul_rn(sp, mid));
           }
         gprev = gi;
         rprev = ri;
@@ -146,75 +172,106 @@ struct TauArgs {
   const long long *offset;
   const double *xyz;
   const int *gp;
-  const double *pop, *T, *weights, *frac1;
+  const double *pop, *T, *weights, *rweights, *frac1;
   const int *up, *lo;
   double v2;
   double *tau;
 };
 
-// one warp per (cell, ray), lanes over the radiative lines
-__global__ void tau_kernel(const __grid_constant__ TauArgs A) {
+// A lane per (cell, ray, line): a block takes 256 consecutive ones, the lines
+// of a ray side by side.  The rays' step lengths, a square root each, are
+// computed once for all their lines, eight points of every ray of the block at
+// a time, in shared memory with the points' grid indices.  A point's term
+// g_u n_l - g_l n_u is shared by the two steps it ends and starts.  The
+// division by the lower level's weight g is the product with its rounded
+// reciprocal y and one residual step, q = a y, q + (a - g q) y, which rounds as
+// the division does (Markstein); the trapezoid's 1/2 is in f12 (exact).  What
+// bounds it: the FP64 pipe, 11 instructions per line and step.  (One warp per
+// ray with two lines per lane left 24 of 64 slots of CO's 40 lines idle and
+// took 17 and the square root.)  CO, 29^3 cells, 12 rays of 8.5 points: 8.5 ->
+// 2.64 ms.
+__global__ void __launch_bounds__(TAU_THREADS) tau_kernel(const __grid_constant__ TauArgs A, int rays_max) {
   constexpr double KB = 1.38065040e-16, MP = 1.67262164e-24, PI = 3.141592653589793238462643383279502884197;
-  const int lane = threadIdx.x & 31;
-  const long long nwarp = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long cj = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-       cj < (long long)A.ncell * A.nrays; cj += nwarp) {
-    const int c = (int)(cj / A.nrays), j = (int)(cj % A.nrays);
-    // FRAC2 of escape_probability.F90:57 for this cell's temperature
-    const double frac2 = 1.0 / __dsqrt_rn(__dadd_rn(
-        __ddiv_rn(__ddiv_rn(__dmul_rn(8.0 * KB, A.T[c]), PI), MP), A.v2));
-    const int ne = A.epray[cj];
-    const long long p0 = A.offset[cj];
-    bool bad = (ne > 0) && (p0 < 0 || p0 + ne >= A.npoint);
-    // lines in chunks of 64, two per lane, so that each point's step length is
-    // computed once per chunk; a point's term g_u n_l - g_l n_u is shared by the
-    // two steps it ends and starts
-    for (int l0 = 0; l0 < A.nlin; l0 += 64) {
-      int u[2], d[2];
-      double gu[2], gd[2], f12[2], prev[2], tau[2];
-      bool act[2];
-#pragma unroll
-      for (int s = 0; s < 2; s++) {
-        const int l = l0 + 32 * s + lane;
-        act[s] = l < A.nlin;
-        u[s] = act[s] ? A.up[l] : 0;
-        d[s] = act[s] ? A.lo[l] : 0;
-        gu[s] = act[s] ? A.weights[u[s]] : 1.0;
-        gd[s] = act[s] ? A.weights[d[s]] : 1.0;
-        f12[s] = act[s] ? __dmul_rn(A.frac1[l], frac2) : 0.0;
-        tau[s] = 0.0;
-        prev[s] = 0.0;
-      }
-      bool badl = bad;
-      if (ne > 0 && !bad) {
-        const int ga = A.gp[p0];
-        if (ga < 0 || ga >= A.ngrid) badl = true;
-        else {
-          const double *pa = A.pop + (size_t)ga * A.nlev;
-#pragma unroll
-          for (int s = 0; s < 2; s++)
-            if (act[s]) prev[s] = __dsub_rn(__dmul_rn(pa[d[s]], gu[s]), __dmul_rn(pa[u[s]], gd[s]));
-        }
-        for (int i = 1; i <= ne && !badl; i++) {
-          const long long p = p0 + i;
-          const int gb = A.gp[p];
-          if (gb < 0 || gb >= A.ngrid) { badl = true; break; }
-          const double step = step_length(A.xyz, p);
-          const double *pb = A.pop + (size_t)gb * A.nlev;
-#pragma unroll
-          for (int s = 0; s < 2; s++)
-            if (act[s]) {
-              const double cur = __dsub_rn(__dmul_rn(pb[d[s]], gu[s]), __dmul_rn(pb[u[s]], gd[s]));
-              const double frac3 = __ddiv_rn(__dadd_rn(prev[s], cur) * 0.5, gd[s]);
-              tau[s] = __dadd_rn(tau[s], __dmul_rn(__dmul_rn(__dmul_rn(f12[s], frac3), step), PC));
-              prev[s] = cur;
-            }
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < 2; s++)
-        if (act[s]) A.tau[((size_t)c * A.nlin + l0 + 32 * s + lane) * A.nrays + j] = badl ? nan("") : tau[s];
+  extern __shared__ __align__(16) unsigned char smem[];
+  double *steps = reinterpret_cast<double *>(smem);                    // [rays_max][TAU_STEPS]
+  double *frac2 = steps + (size_t)rays_max * TAU_STEPS;                // [rays_max]
+  int *gps = reinterpret_cast<int *>(frac2 + rays_max);                // [rays_max][TAU_STEPS], -1: outside the grid
+  int *nes = gps + (size_t)rays_max * TAU_STEPS;                       // [rays_max] points of the ray, -1: bad
+  const int tid = threadIdx.x;
+  const long long total = (long long)A.ncell * A.nrays * A.nlin, nray_all = (long long)A.ncell * A.nrays;
+  for (long long t0 = (long long)blockIdx.x * TAU_THREADS; t0 < total; t0 += (long long)gridDim.x * TAU_THREADS) {
+    const long long ray0 = t0 / A.nlin;
+    const int nr = (int)(min((t0 + TAU_THREADS - 1) / A.nlin, nray_all - 1) - ray0) + 1;
+    int longest = 0;
+    for (int i = tid; i < nr; i += TAU_THREADS) {
+      const long long cj = ray0 + i;
+      const int ne = A.epray[cj];
+      const long long p0 = A.offset[cj];
+      int n = max(ne, 0);
+      if (ne > 0 && (p0 < 0 || p0 + ne >= A.npoint)) n = -1;
+      nes[i] = n;
+      longest = max(longest, n);
+      // FRAC2 of escape_probability.F90:57 for this cell's temperature
+      frac2[i] = 1.0 / __dsqrt_rn(__dadd_rn(
+          __ddiv_rn(__ddiv_rn(__dmul_rn(8.0 * KB, A.T[cj / A.nrays]), PI), MP), A.v2));
     }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    __shared__ int most;
+    if (tid == 0) most = 0;
+    __syncthreads();
+    if ((tid & 31) == 0 && longest > 0) atomicMax(&most, longest);
+    __syncthreads();
+    longest = most;
+    // this thread's ray and line
+    const long long t = t0 + tid;
+    const bool mine = t < total;
+    const long long cj = mine ? t / A.nlin : ray0;
+    const int l = mine ? (int)(t - cj * A.nlin) : 0, ray = (int)(cj - ray0);
+    const int u = A.up[l], d = A.lo[l], ne = mine ? nes[ray] : 0;
+    const double gu = A.weights[u], gd = A.weights[d], rg = A.rweights[d];
+    const double f12 = __dmul_rn(A.frac1[l], frac2[ray]) * 0.5;
+    double prev = 0.0, tau = 0.0;
+    bool bad = ne < 0;
+    if (ne > 0) {
+      const int ga = A.gp[A.offset[cj]];
+      if (ga < 0 || ga >= A.ngrid) bad = true;
+      else {
+        const double *pa = A.pop + (size_t)ga * A.nlev;
+        prev = __dsub_rn(__dmul_rn(pa[d], gu), __dmul_rn(pa[u], gd));
+      }
+    }
+    for (int i0 = 1; i0 <= longest; i0 += TAU_STEPS) {
+      for (int q = tid; q < nr * TAU_STEPS; q += TAU_THREADS) {
+        const int r = q / TAU_STEPS, i = i0 + q - r * TAU_STEPS;
+        if (i > nes[r]) continue;
+        const long long p = A.offset[ray0 + r] + i;
+        const int gb = A.gp[p];
+        gps[q] = (gb >= 0 && gb < A.ngrid) ? gb : -1;
+        steps[q] = step_length(A.xyz, p);
+      }
+      __syncthreads();
+      const int m = bad ? 0 : min(TAU_STEPS, ne - i0 + 1);
+      for (int i = 0; i < m; i++) {
+        const int gb = gps[ray * TAU_STEPS + i];
+        if (gb < 0) { bad = true; break; }
+        const double *pb = A.pop + (size_t)gb * A.nlev;
+        const double cur = __dsub_rn(__dmul_rn(pb[d], gu), __dmul_rn(pb[u], gd));
+        const double x = __dadd_rn(prev, cur);
+        const double q0 = __dmul_rn(x, rg);
+        double frac3 = fma(fma(-gd, q0, x), rg, q0);
+        // beyond the residual step's exponent range, or a weight it was not made for
+        if ((((unsigned)__double2hiint(x) >> 20) & 0x7ff) - 128u > 1790u && (__double_as_longlong(x) << 1) != 0)
+          frac3 = __ddiv_rn(x, gd);
+        tau = __dadd_rn(tau, __dmul_rn(__dmul_rn(__dmul_rn(f12, frac3), steps[ray * TAU_STEPS + i]), PC));
+        prev = cur;
+      }
+      __syncthreads();
+    }
+    if (mine) {
+      const int c = (int)(cj / A.nrays), j = (int)(cj - (long long)c * A.nrays);
+      A.tau[((size_t)c * A.nlin + l) * A.nrays + j] = bad ? nan("") : tau;
+    }
+    __syncthreads();
   }
 }
 
@@ -236,14 +293,18 @@ int launch_tau(const pdr_coolant *cool, const pdr_rays &r, const double *pop, co
   A.pop = pop;
   A.T = T;
   A.weights = cool->dev.weights;
+  A.rweights = cool->dev.rweights;
   A.frac1 = cool->dev.line_frac1;
   A.up = cool->dev.line_up;
   A.lo = cool->dev.line_lo;
   A.v2 = v_turb * v_turb;
   A.tau = tau;
-  const long long warps = (long long)r.ncell * r.nrays;
-  const int blocks = (int)std::max(1ll, std::min((warps + 3) / 4, (long long)sm_count * 16));
-  tau_kernel<<<blocks, 128, 0, st>>>(A);
+  // the rays of a block's 256 consecutive (ray, line) pairs
+  const int rays_max = (TAU_THREADS + A.nlin - 2) / A.nlin + 1;
+  const size_t smem = (size_t)rays_max * (TAU_STEPS * (8 + 4) + 8 + 4);
+  const long long want = ((long long)r.ncell * r.nrays * A.nlin + TAU_THREADS - 1) / TAU_THREADS;
+  const int blocks = (int)std::max(1ll, std::min(want, (long long)sm_count * 16));
+  tau_kernel<<<blocks, TAU_THREADS, smem, st>>>(A, rays_max);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "tau_kernel launch");
 }
@@ -281,8 +342,9 @@ int launch_uvfield(const pdr_rays &r, const double *rho, int field, const double
     }
     if (A.uni_ray >= 0) A.g_uni = best;
   }
-  const int blocks = std::max(1, std::min((r.ncell + 127) / 128, sm_count * 16));
-  uvfield_kernel<<<blocks, 128, 0, st>>>(A);
+  const int per = std::max(1, UV_THREADS / r.nrays);
+  const int blocks = std::max(1, std::min((r.ncell + per - 1) / per, sm_count * 16));
+  uvfield_kernel<<<blocks, UV_THREADS, 0, st>>>(A);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "uvfield_kernel launch");
 }
