@@ -166,9 +166,15 @@ __device__ __forceinline__ bool level_moved_fp64(double sv, double pv, double fl
 // |dL|/2 and |dL|.  The relative change 2|s-p|/(s+p) = 2 tanh(|ln s - ln p|/2)
 // exceeds 1e-2 exactly when |ln s - ln p| > 0.01000008, so |dL| <= 0.0099
 // means "not moved" and |dL| >= 0.0202 means "moved", with margins far beyond
-// the FP64 rounding of the reference's expression.  Everything else -- the
-// band between, zeros, negatives, subnormals, infinities, NaN -- takes the
-// FP64 path.  Positive s passes s >= floor exactly when its bits are >= the
+// the FP64 rounding of the reference's expression.  Between them s and p are
+// within 2.1 % of each other, and FP32 decides: with both truncated to 24 bits
+// relative to s's binade their difference is exact in FP32 and at most 2^-22
+// from s - p, which is 2.4e-5 of the threshold 0.005 (s + p) >= 0.0099, so a
+// difference 6e-5 beside the threshold is on the right side of it.  (Populations
+// of a maturing iteration change by about a per cent: most lie in that band,
+// and the FP64 division of each took three quarters of the kernel's time.)
+// Everything else -- the sliver around the threshold, zeros, negatives,
+// subnormals, infinities, NaN -- takes the FP64 path.  Positive s passes s >= floor exactly when its bits are >= the
 // floor's for floor > 0, always for floor <= 0, never for a NaN floor.
 __device__ __forceinline__ bool level_moved(double sv, double pv, double floor) {
   constexpr unsigned long long MIN_NORMAL = 0x0010000000000000ull, INF = 0x7FF0000000000000ull;
@@ -184,6 +190,11 @@ __device__ __forceinline__ bool level_moved(double sv, double pv, double floor) 
     const long long ad = d < 0 ? -d : d;
     if (ad <= NOT_MOVED) return false;
     if (ad >= MOVED) return true;
+    const float sf = __uint_as_float((unsigned)(sb >> 29 & 0x7fffffull) | 0x3f800000u);
+    const float pf = __uint_as_float((unsigned)((long long)(pb - (sb & INF)) >> 29) + 0x3f800000u);
+    const float diff = fabsf(sf - pf), limit = 0.005f * (sf + pf);
+    if (diff > limit * 1.00006f) return true;
+    if (diff < limit * 0.99994f) return false;
   }
   return level_moved_fp64(sv, pv, floor);
 }
