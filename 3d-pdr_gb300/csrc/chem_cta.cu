@@ -95,7 +95,7 @@ __host__ __device__ inline CtaLayout cta_layout(const WarpTables &T, int ld, siz
   size_t scr = (size_t)nreac * (8 > 2 * mt ? 8 : 2 * mt);
   if (8 * (size_t)T.nop > scr) scr = 8 * (size_t)T.nop;
   L.scr = o; o += al16(scr);
-  L.xs = o; o += al16(8 * (size_t)(n + 2));
+  L.xs = o; o += sp ? 0 : al16(8 * (size_t)(n + 2));   // slot values of the dense forms' assembly
   L.part = o; o += al16(8 * (size_t)(nparts + 1));
   L.red = o; o += al16(2 * MAXW * (8 + 8 + 4));   // sums, argmax keys, argmax rows
   L.sig = o; o += al16(4 * (size_t)(T.neq + 2) * 2);   // column scales, then the FP32 slot values
@@ -606,7 +606,6 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     const WarpTables &T = A.tab;
     const auto &Q = T.sp;
     const int G = T.lanes;
-    if (owns) xs[tid] = yv;
     const float y32 = (float)yv;
     ssc32 = fmaf(this->rtol32, fabsf(y32), this->atol32);
     wsc32 = __frcp_rn(ssc32);
@@ -888,7 +887,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     cx = owns ? __ldg(&A.tab.xe_coef[tid]) : 0.0;
     load_rates(A.rate + (size_t)cell * A.nreac, A.density[cell]);
     if (tid == 0) {
-      xs[n + 1] = 1.0;
+      if (!SP) xs[n + 1] = 1.0;
       xs32[n + 1] = 1.0f;
       part[A.tab.nparts] = 0.0;
       sig[n] = 1.0f;
