@@ -28,6 +28,17 @@
 //        blocks of L and U are inverted in place at setup, so a block step is
 //        a 32x32 product by one warp plus a rank-32 update by the row owners.
 //
+// What bounds it: latency.  Two blocks fit an SM (99 KB of shared memory and
+// 128 registers for the full network's mixed form), a third of the warps wait
+// at a barrier, and the FP64 pipe is busy a quarter of the time.  So the tables'
+// words are fetched ahead of their use, the reads of a group are issued before
+// its stores (the compiler cannot tell the arrays apart), work that one thread
+// or row had to itself is spread over the block, and the loops stay rolled: the
+// kernel had 388 KB of code, three times the instruction cache (now 232 KB).
+// Full network, mixed, cycles per call before and now: right-hand side 46k and
+// 26k; setup 535k and 296k (assembly 62k and 37k, leaf columns 179k and 80k,
+// dense block 171k and 145k, inversion 58k and 34k); 900 cells 416 ms and 358 ms.
+//
 // The matrix is column-major, element (i, j) at j*ld + i with ld odd: thread
 // i's accesses to its own row are consecutive across a warp (coalesced in
 // global memory, conflict-free in shared memory) and the pivot-row reads are
@@ -78,7 +89,7 @@ struct CtaArgs {
 
 // byte offsets of the block's shared arrays (host and device agree)
 struct CtaLayout {
-  size_t scr, xs, part, red, sig, perm, cols, bsv, ys, upan, ws, mat, dinv, yv, rfs, idx, wv, total;
+  size_t scr, xs, part, red, sig, perm, cols, bsv, ys, upan, ws, mat, dinv, yv, rfs, idx, total;
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -87,12 +98,12 @@ __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15)
 // the dense routines on its m x m trailing block)
 __host__ __device__ inline CtaLayout cta_layout(const WarpTables &T, int ld, size_t mt, bool mat_smem,
                                                 bool sp = false) {
-  const int nreac = T.nreac, nparts = T.nparts, G = T.lanes;
+  const int nparts = T.nparts, G = T.lanes;
   const int n = sp ? T.sp.m : T.neq;   // order of the dense matrix
   CtaLayout L;
   size_t o = 0;
   // scr: the RHS operands (FP64) or the two Jacobian scatter buffers
-  size_t scr = (size_t)nreac * (8 > 2 * mt ? 8 : 2 * mt);
+  size_t scr = (size_t)T.nreac * (8 > 2 * mt ? 8 : 2 * mt);
   if (8 * (size_t)T.nop > scr) scr = 8 * (size_t)T.nop;
   L.scr = o; o += al16(scr);
   L.xs = o; o += sp ? 0 : al16(8 * (size_t)(n + 2));   // slot values of the dense forms' assembly
@@ -100,7 +111,8 @@ __host__ __device__ inline CtaLayout cta_layout(const WarpTables &T, int ld, siz
   L.red = o; o += al16(2 * MAXW * (8 + 8 + 4));   // sums, argmax keys, argmax rows
   L.sig = o; o += al16(4 * (size_t)(T.neq + 2) * 2);   // column scales, then the FP32 slot values
   L.perm = o; o += al16(4 * (size_t)n);
-  L.cols = o; o += al16(4 * (size_t)(n + MAXW));   // nonzero U columns of a panel, per-warp counts
+  // nonzero U columns of a panel, per-warp counts, the rows' pivot steps
+  L.cols = o; o += al16(4 * (size_t)((sp ? n : T.neq) + MAXW + (sp ? n + 1 : 0)));
   L.bsv = o; o += al16(mt * (size_t)G);
   L.ys = o; o += al16(mt * (size_t)(n + DB));
   // LU panel; also the assembly's boundary slots (at most 2G - 2)
@@ -108,19 +120,18 @@ __host__ __device__ inline CtaLayout cta_layout(const WarpTables &T, int ld, siz
   L.ws = o; o += al16(sizeof(CoefShared));
   L.mat = o;
   if (sp) {
-    o += al16(mt * (size_t)T.sp.total);
+    o += al16(mt * (size_t)(T.sp.total + 1));   // and a zero
     L.dinv = o; o += al16(mt * (size_t)(T.sp.a > 0 ? T.sp.a : 1));
     L.yv = o; o += al16(mt * (size_t)T.sp.N);
     L.rfs = o; o += al16(4 * (size_t)T.sp.N);
-    // the index tables (a_col, b_col, a_ptr, a_diag, b_ptr, iperm, ul_rows)
-    // and one scatter row per warp
+    // the index tables (a_col, b_col, a_ptr, a_diag, b_ptr, iperm, ul_rows, lev_ptr, ul_ptr)
     L.idx = o;
     o += al16(2 * (size_t)T.sp.off_ba) + al16(2 * (size_t)T.sp.nnz_b) + al16(4 * (size_t)(T.sp.a + 1)) +
-         al16(4 * (size_t)T.sp.a) + al16(4 * (size_t)(T.sp.m + 1)) + al16(4 * (size_t)T.sp.N) + al16(4 * (size_t)T.sp.a);
-    L.wv = o; o += al16(mt * (size_t)MAXW * T.sp.N);
+         al16(4 * (size_t)T.sp.a) + al16(4 * (size_t)(T.sp.m + 1)) + al16(4 * (size_t)T.sp.N) + al16(4 * (size_t)T.sp.a) +
+         al16(4 * (size_t)(T.sp.nlev + 1)) + al16(4 * (size_t)(T.sp.nul + 1));
   } else {
     if (mat_smem) o += al16(mt * (size_t)(n + 2) * ld);
-    L.dinv = L.yv = L.rfs = L.idx = L.wv = o;
+    L.dinv = L.yv = L.rfs = L.idx = o;
   }
   L.total = o;
   return L;
@@ -169,7 +180,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
   // sparse: the index tables, copied to shared memory at the start
   const unsigned short *sa_col = nullptr, *sb_col = nullptr;
   const int *sa_ptr = nullptr, *sa_diag = nullptr, *sb_ptr = nullptr, *siperm = nullptr, *sul_rows = nullptr;
-  MT *wv = nullptr;      // sparse: [MAXW][N] one scatter row per warp
+  const int *slev = nullptr, *sul = nullptr;
   const double inv_n;
   double *kn;            // global, this block's slot
   double *scr, *xs, *part;
@@ -202,7 +213,9 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     if (lane == 0) r[warp] = v;
     __syncthreads();
     double s = 0.0;
-    for (int w = 0; w < nw; w++) s += r[w];
+#pragma unroll
+    for (int w = 0; w < MAXW; w++)
+      if (w < nw) s += r[w];
     return s;
   }
   __device__ __forceinline__ float sum_all(float v) {
@@ -212,7 +225,9 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     if (lane == 0) r[warp] = v;
     __syncthreads();
     float s = 0.0f;
-    for (int w = 0; w < nw; w++) s += r[w];
+#pragma unroll
+    for (int w = 0; w < MAXW; w++)
+      if (w < nw) s += r[w];
     return s;
   }
   __device__ __forceinline__ double max_all(double v) {
@@ -222,6 +237,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     if (lane == 0) r[warp] = v;
     __syncthreads();
     double s = r[0];
+#pragma unroll 1
     for (int w = 1; w < nw; w++) s = fmax(s, r[w]);
     return s;
   }
@@ -242,6 +258,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     __syncthreads();
     unsigned long long best = 0ull;
     int row = -1;
+#pragma unroll 1
     for (int w = 0; w < nw; w++)
       if (rk[w] > best) { best = rk[w]; row = ri[w]; }
     return row;
@@ -289,15 +306,36 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
       P[n + 2 + p] = (ab.x == n ? xe : P[ab.x]) * (ab.y == n ? xe : P[ab.y]);
     }
     __syncthreads();
+    // the terms in groups of four, every read of a group before its stores
+    // (the compiler cannot tell the partial sums from the operands), the next
+    // group's descriptors before this group's rate constants are waited for
     double s = 0.0;
-#pragma unroll 4
-    for (int t = 0; t < T.rhs_len; t++) {
-      const int2 d = __ldg(&T.rhs_t[t * G + tid]);
-      const double k = kn[d.x & 0xffff];
-      const double ks = __hiloint2double(__double2hiint(k) ^ (d.y & (int)0x80000000u), __double2loint(k));
-      s = fma(ks, P[d.y & 0x7fffffff], s);
-      const int fl = (int)((unsigned)d.x >> 16) - 1;
-      if (fl >= 0) { part[fl] = s; s = 0.0; }
+    constexpr int U = 4;
+    int2 d[U];
+    auto fetch = [&](int t) {
+#pragma unroll
+      for (int u = 0; u < U; u++) d[u] = __ldg(&T.rhs_t[min(t + u, T.rhs_len - 1) * G + tid]);
+    };
+    if (T.rhs_len > 0) fetch(0);
+#pragma unroll 1
+    for (int t = 0; t < T.rhs_len; t += U) {
+      double k[U], o[U];
+      int fl[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const double v = kn[d[u].x & 0xffff];
+        o[u] = P[d[u].y & 0x7fffffff];
+        k[u] = __hiloint2double(__double2hiint(v) ^ (d[u].y & (int)0x80000000u), __double2loint(v));
+        fl[u] = (int)((unsigned)d[u].x >> 16) - 1;
+      }
+      fetch(t + U);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (t + u < T.rhs_len) {
+          s = fma(k[u], o[u], s);
+          if (fl[u] >= 0) { part[fl[u]] = s; s = 0.0; }
+        }
+      }
     }
     __syncthreads();
     double f = 0.0;
@@ -422,11 +460,100 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     }
   }
 
+  // One panel of the dense LU by the first warp, for orders up to 96: lane i
+  // keeps the panel entries of rows i, i + 32 and i + 64 in registers, so that a
+  // pivot column costs a warp's argmax and shuffles instead of a block barrier
+  // and a reduction through shared memory.  `mine` holds the lane's rows that
+  // are not pivoted yet; steps[row] = pivot step.  The updates are the block's.
+  __device__ __forceinline__ bool panel_warp(int k0, int kb, unsigned &mine, int *steps) {
+    constexpr int R = 3;
+    MT r[R][PB];
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < R; q++)
+#pragma unroll
+      for (int t = 0; t < PB; t++) r[q][t] = (lane + 32 * q < dn && t < kb) ? M(lane + 32 * q, k0 + t) : MT(0);
+#pragma unroll
+    for (int t = 0; t < PB; t++) {
+      if (t < kb) {
+        unsigned key[R], top = 0u;
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          key[q] = (mine >> q & 1u) ? __float_as_uint(fabsf((float)r[q][t])) : 0u;
+          top = max(top, key[q]);
+        }
+        top = __reduce_max_sync(FULL, top);
+        int p = 0;
+        bool found = false;
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          const unsigned b = __ballot_sync(FULL, (mine >> q & 1u) && key[q] == top);
+          if (!found && b) { p = 32 * q + __ffs(b) - 1; found = true; }
+        }
+        ok = ok && top != 0u;
+        MT u[PB];
+#pragma unroll
+        for (int j = t; j < PB; j++) {
+          const MT v = p >= 64 ? r[2][j] : (p >= 32 ? r[1][j] : r[0][j]);
+          u[j] = __shfl_sync(FULL, v, p & 31);
+        }
+        const MT rinv = rcp(u[t]);
+        if (lane == (p & 31)) {
+          mine &= ~(1u << (p >> 5));
+          steps[p] = k0 + t;
+          perm[k0 + t] = p;
+        }
+#pragma unroll
+        for (int q = 0; q < R; q++)
+          if (mine >> q & 1u) {
+            r[q][t] = r[q][t] * rinv;
+#pragma unroll
+            for (int j = t + 1; j < PB; j++) r[q][j] = fma(-r[q][t], u[j], r[q][j]);
+          }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; q++)
+#pragma unroll
+      for (int t = 0; t < PB; t++)
+        if (lane + 32 * q < dn && t < kb) M(lane + 32 * q, k0 + t) = r[q][t];
+    return ok;
+  }
+
   // LU with partial pivoting in place; false if a column has no nonzero pivot
   __device__ __forceinline__ bool lu() {
     mystep = (tid < dn) ? -1 : dn;
+    const bool by_warp = SP && dn <= 96;
+    int *steps = cnt + MAXW;   // by_warp: the pivot step of each row, then whether all were found
+    unsigned mine = 0u;       // by_warp, first warp: this lane's rows without a pivot
+    // by_warp: the trailing update's rows once per group of warps, the groups
+    // taking the columns in turn
+    const int rows32 = by_warp ? (dn + 31) & ~31 : (int)blockDim.x;
+    const int ngrp = (int)blockDim.x / rows32, ugrp = tid / rows32;
+    const int urow = ugrp < ngrp ? tid - ugrp * rows32 : dn;
+    if (by_warp) {
+      for (int q = 0; q < 3; q++)
+        if (lane + 32 * q < dn) mine |= 1u << q;
+      if (tid < dn) steps[tid] = -1;
+      if (tid == 0) steps[dn] = 1;   // cleared when a panel finds no pivot
+      __syncthreads();
+    }
+#pragma unroll 1
     for (int k0 = 0; k0 < dn; k0 += PB) {
       const int kb = min(PB, dn - k0);
+      if (by_warp) {
+        if constexpr (SP) {
+          __syncthreads();   // the other warps' trailing updates
+          if (warp == 0) {
+            const bool ok = panel_warp(k0, kb, mine, steps);
+            if (lane == 0 && !ok) steps[dn] = 0;
+          }
+        }
+        __syncthreads();
+        if (!steps[dn]) return false;
+        if (tid < dn) mystep = steps[tid];
+      } else
+#pragma unroll 1
       for (int t = 0; t < kb; t++) {
         const int k = k0 + t;
         const bool cand = (mystep < 0);
@@ -437,6 +564,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
         if (mystep < 0) {
           const MT l = M(tid, k) * rinv;
           M(tid, k) = l;
+#pragma unroll 1
           for (int j = k + 1; j < k0 + kb; j++) M(tid, j) = fma(-l, M(p, j), M(tid, j));
         }
       }
@@ -469,6 +597,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
       if (lane == 0) cnt[warp] = __popc(bal);
       __syncthreads();
       int base = 0, ncols = 0;
+#pragma unroll 1
       for (int w = 0; w < nw; w++) {
         const int c = cnt[w];
         base += (w < warp) ? c : 0;
@@ -476,12 +605,12 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
       }
       if (nzc) cols[base + __popc(bal & ((1u << lane) - 1u))] = j;
       __syncthreads();
-      if (mystep < 0) {
+      if (by_warp ? urow < dn && steps[urow] < 0 : mystep < 0) {
         MT l[PB];
         bool any = false;
 #pragma unroll
         for (int t = 0; t < PB; t++) {
-          l[t] = (t < kb) ? M(tid, k0 + t) : MT(0);
+          l[t] = (t < kb) ? M(urow, k0 + t) : MT(0);
           any |= (l[t] != MT(0));
         }
         if (any) {
@@ -489,30 +618,34 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
           // any store (the compiler cannot prove the panel buffer and the
           // matrix apart), the U entries of a column as 16-byte vectors
           constexpr int CB = 4;
-          int c = 0;
-          for (; c + CB <= ncols; c += CB) {
+#pragma unroll 1
+          for (int c = CB * ugrp; c < ncols; c += CB * ngrp) {
+            if (c + CB <= ncols) {
             int jj[CB];
             MT s[CB], u[CB][PB];
 #pragma unroll
             for (int b = 0; b < CB; b++) {
               jj[b] = cols[c + b];
-              s[b] = M(tid, jj[b]);
+              s[b] = M(urow, jj[b]);
               load_upan(jj[b], u[b]);
             }
 #pragma unroll
             for (int b = 0; b < CB; b++) {
 #pragma unroll
               for (int t = 0; t < PB; t++) s[b] = fma(-l[t], u[b][t], s[b]);
-              M(tid, jj[b]) = s[b];
+              M(urow, jj[b]) = s[b];
             }
-          }
-          for (; c < ncols; c++) {
-            const int jj = cols[c];
-            MT s = M(tid, jj), u[PB];
-            load_upan(jj, u);
+            } else {
+#pragma unroll 1
+              for (int e = c; e < ncols; e++) {
+                const int jj = cols[e];
+                MT s = M(urow, jj), u[PB];
+                load_upan(jj, u);
 #pragma unroll
-            for (int t = 0; t < PB; t++) s = fma(-l[t], u[t], s);
-            M(tid, jj) = s;
+                for (int t = 0; t < PB; t++) s = fma(-l[t], u[t], s);
+                M(urow, jj) = s;
+              }
+            }
           }
         }
       }
@@ -521,8 +654,59 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     return true;
   }
 
-  // invert the 32x32 diagonal blocks of L (unit lower) and U in place
-  __device__ __forceinline__ void invert_diagonal_blocks() {
+  // L: lane r holds row r of the inverse; row m is final once the rows above it
+  // have been taken off, and is then handed to the rows below
+  __device__ __forceinline__ void invert_lower(int k0, int bs, int pl) {
+    MT x[DB];
+#pragma unroll
+    for (int t = 0; t < DB; t++) x[t] = (t == lane) ? MT(1) : MT(0);
+#pragma unroll 1
+    for (int m = 0; m + 1 < bs; m++) {
+      const bool below = lane > m && lane < bs;
+      const MT l = below ? M(pl, k0 + m) : MT(0);
+#pragma unroll
+      for (int t = 0; t < DB; t++) {
+        const MT xm = __shfl_sync(FULL, x[t], m);
+        if (below) x[t] = fma(-l, xm, x[t]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < DB; t++)
+      if (t < lane && lane < bs) M(pl, k0 + t) = x[t];
+  }
+
+  // U: lane t makes column t from the last row up, y_t = 1/U_tt,
+  // y_r = -(sum_{m=r+1}^{t} U_rm y_m) / U_rr; a row replaces the factor's once
+  // every lane has read it
+  __device__ __forceinline__ void invert_upper(int k0, int bs, int pl) {
+    const int t = lane;
+#pragma unroll 1
+    for (int r = bs - 1; r >= 0; r--) {
+      MT *row = &M(__shfl_sync(FULL, pl, r), k0);
+      const MT d = rcp(row[r * dld]);
+      MT s = MT(0);
+#pragma unroll 1
+      for (int m0 = (r + 1) & ~7; m0 < bs; m0 += 8) {
+        MT u[8], y[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int m = m0 + k, pm = __shfl_sync(FULL, pl, m);
+          const bool in = m > r && m <= t && t < bs;
+          u[k] = in ? row[m * dld] : MT(0);
+          y[k] = in ? M(pm, k0 + t) : MT(0);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (m0 + k > r && m0 + k <= t) s = fma(u[k], y[k], s);
+      }
+      __syncwarp();
+      if (t < bs && t >= r) row[t * dld] = (t == r) ? d : -s * d;
+      __syncwarp();
+    }
+  }
+
+  // both, a warp for a block, column by column in registers
+  __device__ __forceinline__ void invert_dense() {
     const int nb = (dn + DB - 1) / DB;
     for (int c = warp; c < nb; c += nw) {
       const int k0 = c * DB, bs = min(DB, dn - k0);
@@ -568,6 +752,29 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
         if (r < bs && t < bs && r <= t) M(perm[k0 + r], k0 + t) = x[r];
     }
     __syncthreads();
+  }
+
+  // invert the 32x32 diagonal blocks of L (unit lower) and U in place.  The
+  // sparse form gives L and U of a block a warp each (they read and write
+  // disjoint triangles) and is rolled over the rows: unrolled, the 2 x 496
+  // products are 64 KB of code that three warps fetched once a setup (full
+  // network: 71k cycles a setup, 34k rolled).  The dense forms stay unrolled:
+  // their FP64 matrix is in L2, where the reads in flight are worth more (200
+  // cells of the full network: 1.68 s unrolled, 1.80 s rolled).
+  __device__ __forceinline__ void invert_diagonal_blocks() {
+    if constexpr (SP) {
+      const int nb = (dn + DB - 1) / DB;
+#pragma unroll 1
+      for (int job = warp; job < 2 * nb; job += nw) {
+        const int k0 = (job >> 1) * DB, bs = min(DB, dn - k0);
+        const int pl = (lane < bs) ? perm[k0 + lane] : 0;
+        if ((job & 1) == 0) invert_lower(k0, bs, pl);
+        else invert_upper(k0, bs, pl);
+      }
+      __syncthreads();
+    } else {
+      invert_dense();
+    }
   }
 
   __device__ __forceinline__ bool setup(double yv) {
@@ -630,25 +837,43 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
       Da[r] = k32 * ((ab.y == n ? xe32 : xs32[ab.y]) * sa);
       Db[r] = k32 * ((ab.x == n ? xe32 : xs32[ab.x]) * sb);
     }
-    for (int e = tid; e < Q.total; e += G) S[e] = MT(0);
+    // the storage and the zero behind it (16-byte aligned, padded to 16 bytes)
+    for (int e = tid; e < (Q.total + 4) / 4; e += G) reinterpret_cast<int4 *>(S)[e] = make_int4(0, 0, 0, 0);
     __syncthreads();
     {
       MT *slots = upan;
       MT s = MT(0);
-#pragma unroll 4
-      for (int t = 0; t < T.hlen; t++) {
-        const int2 xy = __ldg(&T.h_xy[t * G + tid]);
-        const int x = xy.x, y = xy.y;
-        const MT nu = (MT)(x >> 19);
-        const int r = x & 0xffff;
-        s = fma(nu, (x & 0x10000) ? Db[r] : Da[r], s);
-        const int kind = (x >> 17) & 3;
-        if (kind == 1) {
-          S[(unsigned)y >> 16] = s * rfs[y & 0xff];
-          s = MT(0);
-        } else if (kind == 2) {
-          slots[(unsigned)y >> 16] = s;
-          s = MT(0);
+      constexpr int U = 4;
+      int2 nx[U];
+      auto fetch = [&](int t) {
+#pragma unroll
+        for (int u = 0; u < U; u++) nx[u] = __ldg(&T.h_xy[min(t + u, T.hlen - 1) * G + tid]);
+      };
+      if (T.hlen > 0) fetch(0);
+#pragma unroll 1
+      for (int t = 0; t < T.hlen; t += U) {
+        int2 xy[U];
+        MT d[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          xy[u] = nx[u];
+          d[u] = ((xy[u].x & 0x10000) ? Db : Da)[xy[u].x & 0xffff];
+        }
+        fetch(t + U);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (t + u < T.hlen) {
+            const int x = xy[u].x, y = xy[u].y;
+            s = fma((MT)(x >> 19), d[u], s);
+            const int kind = (x >> 17) & 3;
+            if (kind == 1) {
+              S[(unsigned)y >> 16] = s * rfs[y & 0xff];
+              s = MT(0);
+            } else if (kind == 2) {
+              slots[(unsigned)y >> 16] = s;
+              s = MT(0);
+            }
+          }
         }
       }
       __syncthreads();
@@ -669,61 +894,63 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     __syncthreads();
   }
 
-  // in place: the leaf rows by dependency level, then the trailing rows'
-  // leaf-column part with its update of the dense block (no pivoting; one
-  // warp per row, the row scattered into the warp's dense row so that every
-  // update finds its entry by column), then the dense block with partial
-  // pivoting.  A row's eliminations run in column order; the updates of one
-  // elimination step go to distinct columns, one per lane.
+  // in place: the leaf columns' elimination from every row, one element per
+  // thread and round (WarpTables::Sparse::g_*; no pivoting), then the dense
+  // block with partial pivoting.  An element takes its products in ascending
+  // elimination order, as a row-by-row elimination would.
+  // A warp per row was bound by its up to 118 eliminations, each a chain of
+  // four dependent shared-memory reads and a row of updates; here every thread
+  // has independent work and a product is two reads and an FMA (full network:
+  // 179k cycles a setup against 80k).
   __device__ __forceinline__ bool sparse_lu() {
     const auto &Q = A.tab.sp;
-    const int a = Q.a;
-    MT *w = wv + (size_t)warp * Q.N;
+    const int G = A.tab.lanes;
     bool ok = true;
-    for (int l = 0; l < Q.nlev; l++) {
-      const int r1 = __ldg(&Q.lev_ptr[l + 1]);
-      for (int r = __ldg(&Q.lev_ptr[l]) + warp; r < r1; r += nw) {
-        const int p0 = sa_ptr[r], pd = sa_diag[r], p1 = sa_ptr[r + 1];
-        for (int p = p0 + lane; p < p1; p += 32) w[sa_col[p]] = S[p];
-        __syncwarp();
-        for (int p = p0; p < pd; p++) {
-          const int k = sa_col[p];
-          const MT lk = w[k] * dinv[k];
-          const int u1 = sa_ptr[k + 1];
-          for (int u = sa_diag[k] + 1 + lane; u < u1; u += 32) {
-            const int j = sa_col[u];
-            w[j] = fma(-lk, S[u], w[j]);
-          }
-          if (lane == 0) S[p] = lk;
-          __syncwarp();
-        }
-        for (int p = pd + lane; p < p1; p += 32) S[p] = w[sa_col[p]];
-        if (lane == 0) {
-          const MT d = w[r];
-          ok &= (d != MT(0));
-          dinv[r] = rcp(d);
-        }
-        __syncwarp();
-      }
-      __syncthreads();
+    // the tables come from L2: the words of a group, its descriptor and a
+    // round's elements are fetched one or two steps ahead
+    const unsigned *pr = Q.g_prod + tid;
+    const int2 *pe = Q.g_elem + tid;
+    unsigned w[4], wn[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      w[k] = __ldg(pr + k * G);
+      wn[k] = __ldg(pr + (4 + k) * G);
     }
-    const int off_ba = Q.off_ba;
-    MT *D = S + Q.off_d;
-    for (int t = warp; t < Q.m; t += nw) {
-      const int p0 = sb_ptr[t], p1 = sb_ptr[t + 1];
-      for (int p = p0 + lane; p < p1; p += 32) w[sb_col[p]] = S[off_ba + p];
-      __syncwarp();
-      for (int p = p0; p < p1; p++) {
-        const int k = sb_col[p];
-        const MT lk = w[k] * dinv[k];
-        const int u1 = sa_ptr[k + 1];
-        for (int u = sa_diag[k] + 1 + lane; u < u1; u += 32) {
-          const int j = sa_col[u];
-          MT &dst = (j < a) ? w[j] : D[(size_t)(j - a) * Q.ldb + t];
-          dst = fma(-lk, S[u], dst);
+    int2 el = __ldg(pe), eln = __ldg(pe + G);
+    int desc = __ldg(&Q.g_group[0]), descn = __ldg(&Q.g_group[1]);
+    MT s = S[el.x & 0xffff];
+#pragma unroll 1
+    for (int g = 0; g < Q.ngroup; g++) {
+      MT l[4], u[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        l[k] = S[w[k] & 0xffff];
+        u[k] = S[w[k] >> 16];
+      }
+      const int here = desc;
+      desc = descn;
+      descn = __ldg(&Q.g_group[min(g + 2, Q.ngroup + 1)]);
+      pr += 4 * G;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        w[k] = wn[k];
+        wn[k] = __ldg(pr + (4 + k) * G);   // the table ends two groups later
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) s = fma(-l[k], u[k], s);
+      if (here & 1) {
+        const int kind = el.x >> 16;
+        if (kind == 3) s *= dinv[el.y];
+        if (kind == 2) {
+          ok &= (s != MT(0));
+          dinv[el.y] = rcp(s);
         }
-        if (lane == 0) S[off_ba + p] = lk;
-        __syncwarp();
+        if (kind) S[el.x & 0xffff] = s;
+        if (here & 2) __syncthreads();
+        pe += G;
+        el = eln;
+        eln = __ldg(pe + (pe + G < Q.g_elem + (size_t)(Q.nround + 1) * G ? G : 0));
+        s = S[el.x & 0xffff];
       }
     }
     if (!__syncthreads_and(ok)) return false;
@@ -738,9 +965,10 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     if (tid == 0) yv[siperm[n]] = MT(0);
     __syncthreads();
     // forward, leaf rows
+#pragma unroll 1
     for (int l = 0; l < Q.nlev; l++) {
-      const int r1 = __ldg(&Q.lev_ptr[l + 1]);
-      for (int r = __ldg(&Q.lev_ptr[l]) + tid; r < r1; r += blockDim.x) {
+      const int r1 = slev[l + 1];
+      for (int r = slev[l] + tid; r < r1; r += blockDim.x) {
         MT s = yv[r];
         const int pd = sa_diag[r];
         for (int p = sa_ptr[r]; p < pd; p++) s = fma(-S[p], yv[sa_col[p]], s);
@@ -760,9 +988,10 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     if (tid < Q.m) yv[a + tid] = xt;
     __syncthreads();
     // backward, leaf rows by U-dependency level
+#pragma unroll 1
     for (int l = 0; l < Q.nul; l++) {
-      const int i1 = __ldg(&Q.ul_ptr[l + 1]);
-      for (int i = __ldg(&Q.ul_ptr[l]) + tid; i < i1; i += blockDim.x) {
+      const int i1 = sul[l + 1];
+      for (int i = sul[l] + tid; i < i1; i += blockDim.x) {
         const int r = sul_rows[i];
         MT s = yv[r];
         const int pd = sa_diag[r], p1 = sa_ptr[r + 1];
@@ -788,12 +1017,17 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     int *bp = reinterpret_cast<int *>(take(4 * (size_t)(Q.m + 1)));
     int *ip = reinterpret_cast<int *>(take(4 * (size_t)Q.N));
     int *ur = reinterpret_cast<int *>(take(4 * (size_t)Q.a));
+    int *lv = reinterpret_cast<int *>(take(4 * (size_t)(Q.nlev + 1)));
+    int *ul = reinterpret_cast<int *>(take(4 * (size_t)(Q.nul + 1)));
     for (int i = tid; i < Q.off_ba; i += blockDim.x) ac[i] = __ldg(&Q.a_col[i]);
     for (int i = tid; i < Q.nnz_b; i += blockDim.x) bc[i] = __ldg(&Q.b_col[i]);
     for (int i = tid; i <= Q.a; i += blockDim.x) ap[i] = __ldg(&Q.a_ptr[i]);
     for (int i = tid; i < Q.a; i += blockDim.x) { ad[i] = __ldg(&Q.a_diag[i]); ur[i] = __ldg(&Q.ul_rows[i]); }
     for (int i = tid; i <= Q.m; i += blockDim.x) bp[i] = __ldg(&Q.b_ptr[i]);
     for (int i = tid; i < Q.N; i += blockDim.x) ip[i] = __ldg(&Q.iperm[i]);
+    for (int i = tid; i <= Q.nlev; i += blockDim.x) lv[i] = __ldg(&Q.lev_ptr[i]);
+    for (int i = tid; i <= Q.nul; i += blockDim.x) ul[i] = __ldg(&Q.ul_ptr[i]);
+    slev = lv; sul = ul;
     sa_col = ac; sb_col = bc; sa_ptr = ap; sa_diag = ad; sb_ptr = bp; siperm = ip; sul_rows = ur;
     __syncthreads();
   }
@@ -821,6 +1055,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     bsv[tid] = v;
     __syncthreads();
     // forward: L y = P b
+#pragma unroll 1
     for (int c = 0; c < nb; c++) {
       const int k0 = c * DB, bs = min(DB, dn - k0);
       if (warp == c % nw) {
@@ -847,6 +1082,7 @@ struct CtaCell : Core<CtaCell<MIXED, SP>, false, MIXED> {
     v = downs ? ys[mystep] : MT(0);
     bsv[tid] = v;
     __syncthreads();
+#pragma unroll 1
     for (int c = nb - 1; c >= 0; c--) {
       const int k0 = c * DB, bs = min(DB, dn - k0);
       if (warp == c % nw) {
@@ -939,7 +1175,7 @@ __global__ void __launch_bounds__(256, SP ? 2 : 1) chem_cta_kernel(const __grid_
   c.xs32 = c.sig + (A.n + 2);
   c.perm = reinterpret_cast<int *>(smem_raw + L.perm);
   c.cols = reinterpret_cast<int *>(smem_raw + L.cols);
-  c.cnt = c.cols + A.n;
+  c.cnt = c.cols + (SP ? A.tab.sp.m : A.n);
   c.bsv = reinterpret_cast<MT *>(smem_raw + L.bsv);
   c.ys = reinterpret_cast<MT *>(smem_raw + L.ys);
   c.upan = reinterpret_cast<MT *>(smem_raw + L.upan);
@@ -955,7 +1191,6 @@ __global__ void __launch_bounds__(256, SP ? 2 : 1) chem_cta_kernel(const __grid_
     c.dmat = c.S + A.tab.sp.off_d;
     c.dn = A.tab.sp.m;
     c.dld = A.tab.sp.ldb;
-    c.wv = reinterpret_cast<MT *>(smem_raw + L.wv);
     c.stage_sparse(smem_raw + L.idx);
   }
   if (total_ptr) total_cells = *total_ptr;

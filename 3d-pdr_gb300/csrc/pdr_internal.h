@@ -115,6 +115,16 @@ struct WarpTables {
     unsigned short *b_col = nullptr;   // their columns, ascending
     int *diag_loc = nullptr;  // [N] storage location of each diagonal entry
     int *e_loc = nullptr;     // [neq] location of (x_e row, species j), -1 where c_j = 0
+    // The elimination of the leaf columns from every row, element by element:
+    // an element's value less its products l u in ascending elimination order,
+    // stored (1), stored with its reciprocal as the pivot of row e.y (2), or
+    // times the reciprocal pivot e.y as a multiplier (3).  Rounds of one element
+    // per thread, the elements of a round with about the same number of
+    // products, padded to groups of four (storage location `total` holds a zero)
+    int nround = 0, ngroup = 0;
+    int *g_group = nullptr;   // [ngroup+2] 1: last group of its round, 2: a block barrier follows it
+    int2 *g_elem = nullptr;   // [nround+1][lanes] location | kind << 16, pivot
+    unsigned *g_prod = nullptr;   // [4 (ngroup+2)][lanes] location of l | location of u << 16
   } sp;
 };
 

@@ -219,6 +219,10 @@ struct SparsePlan {
   int N = 0, a = 0, m = 0, ldb = 0, off_ba = 0, off_d = 0, total = 0;
   std::vector<int> perm, iperm, a_ptr, a_diag, lev_ptr, ul_rows, ul_ptr, b_ptr, diag_loc, e_loc;
   std::vector<unsigned short> a_col, b_col;
+  std::vector<int> g_group;            // the leaf columns' elimination (WarpTables::Sparse)
+  std::vector<int2> g_elem;
+  int nround = 0;
+  std::vector<unsigned> g_prod;
   std::vector<std::bitset<256>> F;   // filled pattern in elimination order
   // storage location of entry (unknown i, unknown j), -1 outside the pattern
   int loc(int i, int j) const {
@@ -404,6 +408,75 @@ static bool sparse_plan(int neq, const std::vector<std::pair<int, int>> &entries
     if (xe[j] != 0) sp.e_loc[j] = sp.loc(sp.iperm[neq], sp.iperm[j]);
   for (int v : sp.diag_loc)
     if (v < 0) return false;
+  return true;
+}
+
+// The rounds of the leaf columns' elimination for G threads.  An element (i, j)
+// needs the factors (i, k) and (k, j) of its products, and a multiplier (i, k)
+// the pivot (k, k): its phase is one after the last of them.  (The leaf rows'
+// dependency levels are not enough: two rows of a level may still meet in a
+// third row's multipliers, through a U entry of one in the other's column.)
+// The dense block's elements, which no leaf column needs, come last.
+static bool gather_plan(SparsePlan &sp, int G) {
+  if (sp.total >= 65535) return false;
+  struct Elem { int loc, kind, piv; std::vector<unsigned> prod; };
+  // element (i, j): its products over the leaf columns k < min(i, j) in ascending order
+  auto element = [&](int i, int j) {
+    Elem e{sp.loc(i, j), 1, 0, {}};
+    for (int k = 0; k < std::min({i, j, sp.a}); k++)
+      if (sp.F[i].test(k) && sp.F[k].test(j)) e.prod.push_back((unsigned)sp.loc(i, k) | ((unsigned)sp.loc(k, j) << 16));
+    return e;
+  };
+  auto emit = [&](std::vector<Elem> &es) {
+    std::stable_sort(es.begin(), es.end(), [](const Elem &x, const Elem &y) { return x.prod.size() > y.prod.size(); });
+    for (size_t b = 0; b < es.size(); b += G) {
+      const size_t groups = std::max<size_t>(1, (es[b].prod.size() + 3) / 4);
+      for (size_t g = 1; g <= groups; g++) sp.g_group.push_back((g == groups ? 1 : 0) | (g == groups && b + G >= es.size() ? 2 : 0));
+      sp.nround++;
+      for (int t = 0; t < G; t++) {
+        const bool live = b + t < es.size();
+        sp.g_elem.push_back(live ? int2{es[b + t].loc | (es[b + t].kind << 16), es[b + t].piv} : int2{sp.total, 0});
+      }
+      for (size_t c = 0; c < 4 * groups; c++)
+        for (int t = 0; t < G; t++)
+          sp.g_prod.push_back(b + t < es.size() && c < es[b + t].prod.size() ? es[b + t].prod[c]
+                                                                                : (unsigned)sp.total * 0x10001u);
+    }
+  };
+  std::vector<std::vector<int>> phase(sp.N, std::vector<int>(sp.N, 0));
+  std::vector<std::vector<Elem>> phases;
+  for (int m = 0; m < sp.a; m++) {
+    auto add = [&](int i, int j, int kind) {
+      if (!sp.F[i].test(j)) return;
+      int ph = kind == 3 ? phase[m][m] + 1 : 0;
+      for (int k = 0; k < m; k++)
+        if (sp.F[i].test(k) && sp.F[k].test(j)) ph = std::max({ph, phase[i][k] + 1, phase[k][j] + 1});
+      phase[i][j] = ph;
+      if ((int)phases.size() <= ph) phases.resize(ph + 1);
+      phases[ph].push_back(element(i, j));
+      phases[ph].back().kind = kind;
+      phases[ph].back().piv = m;
+    };
+    add(m, m, 2);
+    for (int j = m + 1; j < sp.N; j++) add(m, j, 1);
+    for (int i = m + 1; i < sp.N; i++) add(i, m, 3);
+  }
+  // a U entry without products is already what it has to be
+  for (auto &es : phases) {
+    es.erase(std::remove_if(es.begin(), es.end(), [](const Elem &e) { return e.kind == 1 && e.prod.empty(); }), es.end());
+    if (!es.empty()) emit(es);
+  }
+  std::vector<Elem> es;
+  for (int i = sp.a; i < sp.N; i++)
+    for (int j = sp.a; j < sp.N; j++) {
+      Elem e = element(i, j);
+      if (!e.prod.empty()) es.push_back(std::move(e));
+    }
+  emit(es);
+  // the reads run two groups and a round ahead
+  sp.g_group.insert(sp.g_group.end(), 2, 0);
+  sp.g_elem.insert(sp.g_elem.end(), G, int2{sp.total, 0});
+  sp.g_prod.insert(sp.g_prod.end(), (size_t)8 * G, (unsigned)sp.total * 0x10001u);
   return true;
 }
 
@@ -656,7 +729,7 @@ int build_device_tables(pdr_net *net) {
       if (G > kWarp) {
         std::vector<std::pair<int, int>> ent;
         for (auto &x : hs) ent.push_back({x.i, x.col});
-        w.sp.ok = sparse_plan(neq, ent, h.xe, G, plan) ? 1 : 0;
+        w.sp.ok = sparse_plan(neq, ent, h.xe, G, plan) && gather_plan(plan, G) ? 1 : 0;
       }
       auto sp_loc = [&](int i, int col) -> unsigned {
         if (!w.sp.ok) return 0u;
@@ -826,6 +899,11 @@ int build_device_tables(pdr_net *net) {
       d.b_col = upload(net, plan.b_col, rc2);
       d.diag_loc = upload(net, plan.diag_loc, rc2);
       d.e_loc = upload(net, plan.e_loc, rc2);
+      d.nround = plan.nround;
+      d.ngroup = (int)plan.g_group.size() - 2;
+      d.g_group = upload(net, plan.g_group, rc2);
+      d.g_elem = upload(net, plan.g_elem, rc2);
+      d.g_prod = upload(net, plan.g_prod, rc2);
     }
     return rc2;
   };
