@@ -82,9 +82,10 @@ __device__ __forceinline__ double escape_ray(double t) {
                       INF = 0x7ff0000000000000ll;   // 1e-8, 5, 700, infinity
   if (mag < SMALL) return 1.0;
   if (bits < 0 && mag > FIVE && mag <= INF) return (1.0 - exp(5.0)) / (-5.0);
-  if (mag < BIG) return fp64::div_fast(1.0 - fp64::exp_fast(fp64::flip(t)), t);
-  return mag <= 0x7e00000000000000ll ? fp64::div_fast(1.0, t)   // exp(-t) is below half an ulp of 1
-                                     : (1.0 - exp(-t)) / t;
+  if (mag > 0x7e00000000000000ll) return (1.0 - exp(-t)) / t;
+  double num = 1.0;   // from 700 on, exp(-t) is below half an ulp of 1
+  if (mag < BIG) num = 1.0 - fp64::exp_fast(fp64::flip(t));
+  return fp64::div_fast(num, t);   // one division: a warp's lanes have tau on both sides
 }
 
 // exp(x) - 1 > 0 as escape_probability.F90 writes it, for x = h nu / k T
@@ -286,7 +287,8 @@ __device__ __forceinline__ bool refine_ok(double ax, double as, double prev, dou
 // and stored once for four updates; the solves move four columns per round of
 // shuffles.  (The Gauss-Jordan inverse this replaces updated all n^2 entries
 // at each of n steps, one dependent load, FMA and store after the other.)
-// 64,000 CO cells, mixed: 14.9 -> 6.3 ms.
+// 64,000 CO cells, mixed: 14.9 -> 5.8 ms (6.1 before the shared row sums and
+// the separate pass over the radiative entries).
 
 // n4 x n4 factors at a; upan: 4 n4 floats, 16-byte aligned; perm[k] the pivot
 // row of step k, dinv[k] its reciprocal pivot
@@ -443,6 +445,28 @@ __device__ __forceinline__ void lu_pp_solve(const float *a, int n4, int ld, cons
   }
 }
 
+// Sums over the columns of an n x n matrix (n <= 64): s0 of row `lane` and s1
+// of row lane + 32, both taken on from their values at entry; term(i, j, v) is
+// v with the term of (i, j) added.  A lane has a row; the rows from 32 on would
+// leave most lanes idle at full price, so up to four lanes share one of them
+// (CO's 41 rows: 57 FP64 instructions in place of 82).
+template <class Term>
+__device__ __forceinline__ void row_sums(int n, Term term, double &s0, double &s1) {
+  const int lane = threadIdx.x & 31, extra = n - 32;
+  const int i0 = min(lane, n - 1);
+#pragma unroll 4
+  for (int j = 0; j < n; j++) s0 = term(i0, j, s0);
+  if (extra <= 0) return;
+  const int parts = min(4, 32 / extra), len = (n + parts - 1) / parts;
+  const int r = lane / parts, j0 = (lane - r * parts) * len, j1 = min(n, j0 + len);
+  const int i1 = 32 + min(r, extra - 1);
+  double t = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < len; k++)
+    if (j0 + k < j1) t = term(i1, j0 + k, t);
+  for (int k = 0; k < parts; k++) s1 += __shfl_sync(FULL, t, (lane * parts + k) & 31);
+}
+
 template <bool MIXED>
 __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ CoolantTables C,
                                                      const __grid_constant__ LevArgs A) {
@@ -512,14 +536,21 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
 #pragma unroll 2
         for (int e = lane; e < nn; e += 32) {
           double v = fma(fma(__ldg(&df[e]), st, __ldg(&lo[e])), dq, first ? 0.0 : R[e]);
-          if (last) {
-            const int po = nrad ? __ldg(&C.pair_of[e]) : 0;
-            if (po) v = (po > 0 ? radd[po - 1] : radu[-po - 1]) + v;
-            if (mag_bits(v) < 0x358dee7a4ad4b81fll) v = 0.0;   // 1e-50
-          }
+          // the radiative entries get their term, and the threshold, below
+          if (last && !(nrad && __ldg(&C.pair_of[e])) && mag_bits(v) < 0x358dee7a4ad4b81fll) v = 0.0;   // 1e-50
           R[e] = v;
         }
       }
+      __syncwarp();
+      // the radiative entries, two a pair: added as they are made they would
+      // cost nearly every warp of entries an FP64 add
+      if (C.npart > 0)
+        for (int k = lane; k < 2 * nrad; k += 32) {
+          const int pe = k >> 1, ij = C.pair_ij[pe], i = ij & 0xff, j = (ij >> 8) & 0xff;
+          const int e = (k & 1) ? j * n + i : i * n + j;
+          const double v = ((k & 1) ? radu[pe] : radd[pe]) + R[e];
+          R[e] = mag_bits(v) < 0x358dee7a4ad4b81fll ? 0.0 : v;
+        }
       if (C.npart == 0)
         for (int e = lane; e < nn; e += 32) {
           const int po = nrad ? __ldg(&C.pair_of[e]) : 0;
@@ -528,13 +559,15 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
         }
     }
     __syncwarp();
-    // the cooling rate: the line values summed over i > j in row-major order,
-    // as the reference adds them; the non-radiative pairs contribute zeros,
-    // which leave the sum unchanged, so only the radiative pairs are added
-    if (lane == 0) {
+    // the cooling rate: the sum of the line values (the non-radiative pairs
+    // contribute zeros), by all lanes: an FP64 add costs a warp the same
+    // whatever its lanes, and one lane's 40 of CO were a twentieth of the kernel
+    {
       double cool = 0.0;
-      for (int pe = 0; pe < C.nrad; pe++) cool = cool + lines[pe];
-      A.cooling[cell] = cool;
+      for (int pe = lane; pe < C.nrad; pe += 32) cool += lines[pe];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) cool += __shfl_xor_sync(FULL, cool, o);
+      if (lane == 0) A.cooling[cell] = cool;
     }
     if (A.line) {
       double *lo = A.line + (size_t)cell * nn;
@@ -544,10 +577,11 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
     }
     __syncwarp();
     // ---- solvlevpop matrix: transpose, diagonal -sum, conservation row ----
-    for (int i = lane; i < n; i += 32) {
-      double out = 0.0;
-      for (int j = 0; j < n; j++) out = out + R[i * n + j];
-      b[i] = out;
+    {
+      double s0 = 0.0, s1 = 0.0;
+      row_sums(n, [&](int i, int j, double v) { return v + R[i * n + j]; }, s0, s1);
+      if (lane < n) b[lane] = s0;
+      if (lane + 32 < n) b[lane + 32] = s1;
     }
     __syncwarp();
     for (int e = lane; e < nn; e += 32) {
@@ -603,14 +637,7 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
       for (int it = 0; it < 3 && ok && !good; it++) {
         __syncwarp();
         double d0 = lane < n ? b[lane] : 0.0, d1 = lane + 32 < n ? b[lane + 32] : 0.0;
-        const double *q0 = R + (lane < n ? lane : 0) * n, *q1 = R + (lane + 32 < n ? lane + 32 : 0) * n;
-        const bool two = n > 32;
-#pragma unroll 4
-        for (int l = 0; l < n; l++) {
-          const double xl = x[l];
-          d0 = fma(-q0[l], xl, d0);
-          if (two) d1 = fma(-q1[l], xl, d1);
-        }
+        row_sums(n, [&](int i, int l, double v) { return fma(-R[i * n + l], x[l], v); }, d0, d1);
         __syncwarp();
         c0 = lane < n ? (float)d0 * s0 : 0.0f;
         c1 = lane + 32 < n ? (float)d1 * s1 : 0.0f;
@@ -852,7 +879,7 @@ int launch_levpop(const pdr_coolant *c, const LevArgsHost &h, bool mixed, int sm
   A.density = h.density; A.T = h.T; A.Td = h.Td; A.partner5 = h.partner5; A.cdens = h.cdens;
   A.spop = h.spop; A.tau = h.tau; A.pop = h.pop; A.cooling = h.cooling; A.line = h.line; A.status = h.status;
   const int n = c->dev.nlev;
-  if (n > 64) {   // the Gauss-Jordan pivot mask holds 64 levels
+  if (n > 64) {   // the elimination gives a lane two rows at most
     set_error("pdr_levpop_batched: coolants with more than 64 levels are not supported");
     return PDR_E_ARG;
   }
