@@ -11,8 +11,8 @@
 //
 // The work is gathers: per point 3 coordinates, a grid index, the density of
 // that grid point and, for the columns, its abundances.  Threads take one
-// cell (UV field) or one (cell, ray, group of 8 species) (columns) and walk
-// its points sequentially; consecutive threads take consecutive cells (rays),
+// (cell, ray) (UV field) or one (cell, ray, group of 8 species) (columns) and
+// walk its points sequentially; consecutive threads take consecutive rays,
 // whose point lists are adjacent in memory.
 #include <algorithm>
 
