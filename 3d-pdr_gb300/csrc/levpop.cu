@@ -36,30 +36,39 @@ constexpr double PI = 3.141592653589793238462643383279502884197;
 constexpr unsigned FULL = 0xffffffffu;
 
 // per-warp shared memory: the nlev^2 FP64 rate matrix (before it, the rays'
-// escape probabilities), the radiative pairs' line values and rates up and
-// down, four nlev vectors, an int vector and, for the mixed solve, the FP32
-// factors with their panel and pivots
+// escape probabilities), the right-hand side, and one region that has, in turn,
+// the radiative pairs' line values and rates up and down with the current
+// populations, then what the solve needs: the multipliers, the active indices
+// and the solution of the FP64 elimination, or the FP32 factors (beside the
+// solution), whose place the elimination takes again for a cell that is
+// re-solved.  Side by side they were 24.9 KB a warp for CO mixed and 16.3 KB
+// FP64, 9 and 14 warps on an SM; 23.1 and 15.1 KB let 10 and 15: 64,000 cells
+// mixed 5.80 -> 5.27 ms, 20,011 cells FP64 3.25 -> 3.10 ms.
 struct LevLayout {
   size_t R, lines, b, sp, x, rs, act, Mf, upan, total;
 };
 __host__ __device__ inline LevLayout levpop_layout(int n, int nrad, bool mixed) {
   auto al = [](size_t v) { return (v + 15) & ~size_t(15); };
+  auto most = [](size_t p, size_t q) { return p > q ? p : q; };
   LevLayout L;
   size_t o = 0;
   L.R = o; o += al(8 * (size_t)n * n);
-  L.lines = o; o += al(24 * (size_t)(nrad > 0 ? nrad : 1));
   L.b = o; o += al(8 * (size_t)n);
-  L.sp = o; o += al(8 * (size_t)n);
-  L.x = o; o += al(8 * (size_t)n);
-  L.rs = o; o += al(8 * (size_t)n);
-  L.act = o; o += al(4 * (size_t)n);
-  L.Mf = L.upan = o;
+  L.x = o;
+  if (mixed) o += al(8 * (size_t)n);   // kept while the factors and, later, the elimination are in the region
+  L.lines = L.Mf = o;
+  L.sp = L.lines + al(24 * (size_t)(nrad > 0 ? nrad : 1));
+  size_t end = L.sp + al(8 * (size_t)n);
+  L.rs = mixed ? o : L.x + al(8 * (size_t)n);
+  L.act = L.rs + al(8 * (size_t)n);
+  end = most(end, L.act + al(4 * (size_t)n));
+  L.upan = o;
   if (mixed) {
     const size_t n4 = ((size_t)n + 3) & ~size_t(3);
-    o += al(4 * n4 * (n4 | 1));
-    L.upan = o; o += al(4 * 6 * n4);   // the panel, the reciprocal pivots, the pivot order
+    L.upan = L.Mf + al(4 * n4 * (n4 | 1));
+    end = most(end, L.upan + al(4 * 6 * n4));   // the panel, the reciprocal pivots, the pivot order
   }
-  L.total = o;
+  L.total = end;
   return L;
 }
 
@@ -287,8 +296,8 @@ __device__ __forceinline__ bool refine_ok(double ax, double as, double prev, dou
 // and stored once for four updates; the solves move four columns per round of
 // shuffles.  (The Gauss-Jordan inverse this replaces updated all n^2 entries
 // at each of n steps, one dependent load, FMA and store after the other.)
-// 64,000 CO cells, mixed: 14.9 -> 5.8 ms (6.1 before the shared row sums and
-// the separate pass over the radiative entries).
+// 64,000 CO cells, mixed: 14.9 -> 5.3 ms (6.1 before the shared row sums,
+// the separate pass over the radiative entries and the smaller layout).
 
 // n4 x n4 factors at a; upan: 4 n4 floats, 16-byte aligned; perm[k] the pivot
 // row of step k, dinv[k] its reciprocal pivot
