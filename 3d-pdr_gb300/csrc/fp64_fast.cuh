@@ -33,6 +33,8 @@ namespace pdr {
 namespace fp64 {
 
 #include "fp64_tables.inc"
+static_assert(alignof(ExpRow) == alignof(double2), "a row is read with one 16-byte load");
+static_assert(alignof(LogRow) == alignof(float2), "c and lo of a row are read with one 8-byte load");
 
 constexpr double K_LN2 = 1477.3197218702985;        // 1024/ln 2
 constexpr float K_LN2_LO = 2.08438003e-14f;         //   its rounding error

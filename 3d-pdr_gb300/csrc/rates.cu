@@ -19,6 +19,7 @@
 // rates_cell_general, one warp per cell, expression by expression.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include <mutex>
@@ -94,8 +95,9 @@ __host__ __device__ R splint(const R *xa, const R *ya, const R *y2a, int n, R x)
 // splines as bicubic patches (coefficient of x^n y^m at [n][m], x and y from
 // the patch's lower corner in log10 N(CO), log10 N(H2)), and XLAMBDA's cubic
 // pieces over LBAR's range (c0..c3, the piece's start, 1/its width) for the
-// natural spline [0] and the linear variant [1].
-struct ShieldFast {
+// natural spline [0] and the linear variant [1].  (A patch is read with 16-byte
+// loads.)
+struct alignas(16) ShieldFast {
   double patch[7][5][4][4];
   double lam[2][4][6];
 };
@@ -502,6 +504,9 @@ __device__ __forceinline__ double coshield_fast(double u, double w) {
   w = fmin(fmax(w, 18.0), 23.0);
   const int p = min((int)fp64::d2f(u) - 12, 6), q = min((int)fp64::d2f(w) - 18, 4);
   const double x = u - fp64::f2d((float)(p + 12)), y = w - fp64::f2d((float)(q + 18));
+  static_assert(alignof(ShieldFast) % alignof(double2) == 0 && sizeof(d_shield.patch[0][0]) % sizeof(double2) == 0 &&
+                    offsetof(ShieldFast, patch) % alignof(double2) == 0,
+                "a patch is read with 16-byte loads");
   const double2 *K = reinterpret_cast<const double2 *>(d_shield.patch[p][q]);
   double f = 0.0;
 #pragma unroll 1
