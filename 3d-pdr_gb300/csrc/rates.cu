@@ -116,17 +116,17 @@ static void piece(R ya, R yb, R a2, R b2, R h, R *c) {
 #pragma nv_diag_suppress 20208   // the host evaluates these in long double; no device code is made of it
 static void shield_fast_tables(const ShieldTables &t, ShieldFast &f) {
   using R = long double;
-  R nco[8], nh2[6], u[64];
+  R nco[8], nh2[6], u[8];
   for (int i = 0; i < 8; i++) nco[i] = t.nco[i];
   for (int j = 0; j < 6; j++) nh2[j] = t.nh2[j];
-  static R rows[8][5][4];
+  R rows[8][5][4];
   for (int i = 0; i < 8; i++) {
     R row[6], y2[6];
     for (int j = 0; j < 6; j++) row[j] = t.sco[i][j];
     spline_natural<R>(nh2, row, 6, y2, u);
     for (int q = 0; q < 5; q++) piece<R>(row[q], row[q + 1], y2[q], y2[q + 1], R(1), rows[i][q]);
   }
-  static R acc[7][5][4][4];
+  R acc[7][5][4][4];
   for (auto &a : acc) for (auto &b : a) for (auto &c : b) for (R &d : c) d = 0;
   for (int i = 0; i < 8; i++) {
     R e[8], y2[8];
@@ -155,31 +155,41 @@ static void shield_fast_tables(const ShieldTables &t, ShieldFast &f) {
     }
 }
 
-static bool g_shield_ready[64];
-
-int upload_shield_tables(int dev) {
-  if (dev >= 0 && dev < 64 && g_shield_ready[dev]) return 0;
+// the tables of every device, made once per process
+struct ShieldHost {
   ShieldTables t;
-  double u[64];
-  for (int i = 0; i < 30; i++) { t.lgrid[i] = kLGrid[i]; t.xgrid[i] = kXGrid[i]; }
-  spline_natural<double>(t.lgrid, t.xgrid, 30, t.xderiv, u);
-  for (int i = 0; i < 8; i++) t.nco[i] = kNCOGrid[i];
-  for (int j = 0; j < 6; j++) t.nh2[j] = kNH2Grid[j];
-  for (int i = 0; i < 8; i++) {
-    double row[6], y2[6];
-    for (int j = 0; j < 6; j++) { row[j] = kSCO[j][i]; t.sco[i][j] = kSCO[j][i]; }
-    spline_natural<double>(t.nh2, row, 6, y2, u);
-    for (int j = 0; j < 6; j++) t.scoderiv[i][j] = y2[j];
-  }
-  cudaError_t e = cudaMemcpyToSymbol(c_shield, &t, sizeof t);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyToSymbol(shield tables)");
-  {
-    static ShieldFast f;
+  ShieldFast f;
+  ShieldHost() {
+    double u[30];
+    for (int i = 0; i < 30; i++) { t.lgrid[i] = kLGrid[i]; t.xgrid[i] = kXGrid[i]; }
+    spline_natural<double>(t.lgrid, t.xgrid, 30, t.xderiv, u);
+    for (int i = 0; i < 8; i++) t.nco[i] = kNCOGrid[i];
+    for (int j = 0; j < 6; j++) t.nh2[j] = kNH2Grid[j];
+    for (int i = 0; i < 8; i++) {
+      double row[6], y2[6];
+      for (int j = 0; j < 6; j++) { row[j] = kSCO[j][i]; t.sco[i][j] = kSCO[j][i]; }
+      spline_natural<double>(t.nh2, row, 6, y2, u);
+      for (int j = 0; j < 6; j++) t.scoderiv[i][j] = y2[j];
+    }
     shield_fast_tables(t, f);
-    e = cudaMemcpyToSymbol(d_shield, &f, sizeof f);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyToSymbol(shield pieces)");
   }
-  if (dev >= 0 && dev < 64) g_shield_ready[dev] = true;
+};
+
+// Uploads the tables to `dev`, the calling thread's device, at its first call.
+// Any number of threads may make that call: one copies, the others return when
+// the device has the tables, and none copies over tables that are in use.
+int upload_shield_tables(int dev) {
+  static std::mutex mu;
+  static bool ready[64];
+  static const ShieldHost host;
+  std::lock_guard<std::mutex> lk(mu);
+  const bool known = dev >= 0 && dev < 64;
+  if (known && ready[dev]) return 0;
+  cudaError_t e = cudaMemcpyToSymbol(c_shield, &host.t, sizeof host.t);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyToSymbol(shield tables)");
+  e = cudaMemcpyToSymbol(d_shield, &host.f, sizeof host.f);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyToSymbol(shield pieces)");
+  if (known) ready[dev] = true;
   return 0;
 }
 

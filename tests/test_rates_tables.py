@@ -25,6 +25,7 @@ def check(tmp_path_factory):
     return exe
 
 
-def test_alignment(check):
-    r = subprocess.run([check], capture_output=True, text=True, timeout=300)
+@pytest.mark.parametrize("what", ["align", "threads"])
+def test_tables(check, what):
+    r = subprocess.run([check, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
