@@ -432,7 +432,7 @@ struct WarpCell : Core<WarpCell<NSP, MIXED, ZSH>, ZSH, MIXED> {
     }
     double v = xe_term(yv);
     __syncwarp();
-    int d = pk[lane];
+    PairWord d(pk[lane]);
 #pragma unroll 1
     for (int k = 0; k < T.pk_len; k++) {
       const int o = 16 >> k;   // 0 from round 5 on
@@ -440,9 +440,9 @@ struct WarpCell : Core<WarpCell<NSP, MIXED, ZSH>, ZSH, MIXED> {
         if (lane == 0) P[NSP] = v;
         __syncwarp();
       }
-      const double x = P[d & 0xff], y = P[(d >> 8) & 0xff];
-      const int at = d >> 16;
-      d = pk[min(k + 1, T.pk_len - 1) * kWarp + lane];
+      const double x = P[d.a()], y = P[d.b()];
+      const int at = d.operand();
+      d = PairWord(pk[min(k + 1, T.pk_len - 1) * kWarp + lane]);
       const double w = __shfl_down_sync(FULL, v, o);
       const bool sum = lane < o;
       const double r = fma(sum ? v : x, sum ? 1.0 : y, sum ? w : -0.0);
@@ -464,15 +464,15 @@ struct WarpCell : Core<WarpCell<NSP, MIXED, ZSH>, ZSH, MIXED> {
       for (int u = 0; u < 4; u++) d4[u] = (unsigned)rt[(t + u) * kWarp + lane];
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        k[u] = *reinterpret_cast<const double *>(reinterpret_cast<const char *>(kn) + (d4[u] & 0xfff8));
-        o[u] = *reinterpret_cast<const double *>(reinterpret_cast<const char *>(P) + ((d4[u] >> 15) & 0xfff8));
+        k[u] = *reinterpret_cast<const double *>(reinterpret_cast<const char *>(kn) + TermWord(d4[u]).rate_at());
+        o[u] = *reinterpret_cast<const double *>(reinterpret_cast<const char *>(P) + TermWord(d4[u]).operand_at());
       }
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         // nu kn_r with nu = +-1 (|nu| > 1 reads its extra constant): the sign
         // bit of kn_r flipped in the integer pipe
-        s = fma(__hiloint2double(__double2hiint(k[u]) ^ (int)(d4[u] & 0x80000000u), __double2loint(k[u])), o[u], s);
-        if (d4[u] & 1u) {
+        s = fma(__hiloint2double(__double2hiint(k[u]) ^ (int)TermWord(d4[u]).sign(), __double2loint(k[u])), o[u], s);
+        if (TermWord(d4[u]).last()) {
           *pp++ = s;
           s = 0.0;
         }
@@ -561,16 +561,16 @@ struct WarpCell : Core<WarpCell<NSP, MIXED, ZSH>, ZSH, MIXED> {
 #pragma unroll
         for (int u = 0; u < 4; u++) x[u] = ht[(t + u) * kWarp + lane];
 #pragma unroll
-        for (int u = 0; u < 4; u++) d[u] = Da[x[u] & 0x3fff];
+        for (int u = 0; u < 4; u++) d[u] = Da[JacWord(x[u]).index()];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
           // nu, a small signed integer: converted without the FP64 pipe
-          const float nu = (float)((x[u] << 11) >> 27);
+          const float nu = (float)JacWord(x[u]).nu();
           if constexpr (MIXED) s = fmaf(nu, d[u], s);
           else s = fma(fp64::f2d(nu), d[u], s);
-          const int kind = (x[u] >> 14) & 3;
+          const int kind = JacWord(x[u]).kind();
           if (kind) {
-            (kind == 1 ? jrow : slots)[(unsigned)x[u] >> 21] = s;
+            (kind == 1 ? jrow : slots)[JacWord(x[u]).target()] = s;
             s = MT(0);
           }
         }

@@ -24,6 +24,48 @@ enum RateKind {
 
 constexpr int kWarp = 32;
 
+// Words of the warp integrator's packed tables.  The fields hold every network
+// whose per-warp arrays fit a block's shared memory: 8 bytes a rate constant,
+// and with the two scatter buffers 16 to 24 bytes a reaction, of at most 227 KB.
+//
+// a term of the right-hand side
+struct TermWord {
+  static constexpr int MAX_RATE = (1 << 15) - 1, MAX_OPERAND = (1 << 11) - 1;
+  unsigned w;
+  __host__ __device__ explicit TermWord(unsigned word) : w(word) {}
+  __host__ __device__ TermWord(int rate, int operand, bool negative, bool last)
+      : w((unsigned)rate << 3 | (unsigned)operand << 18 | (negative ? 0x80000000u : 0u) | (last ? 1u : 0u)) {}
+  // byte offsets of its rate constant and its operand
+  __host__ __device__ unsigned rate_at() const { return w & 0x3fff8u; }
+  __host__ __device__ unsigned operand_at() const { return (w >> 15) & 0x3ff8u; }
+  __host__ __device__ int rate() const { return (int)(rate_at() >> 3); }
+  __host__ __device__ int operand() const { return (int)(operand_at() >> 3); }
+  __host__ __device__ unsigned sign() const { return w & 0x80000000u; }
+  __host__ __device__ bool negative() const { return sign() != 0u; }
+  __host__ __device__ bool last() const { return (w & 1u) != 0u; }   // the last one of a partial sum
+};
+// a contribution nu dphi_r/dx to an entry of the Jacobian; index: r, plus nreac for the second reactant's
+struct JacWord {
+  static constexpr int MAX_INDEX = (1 << 15) - 1, MIN_NU = -8, MAX_NU = 7, MAX_TARGET = (1 << 11) - 1;
+  int w;
+  __host__ __device__ explicit JacWord(int word) : w(word) {}
+  __host__ __device__ JacWord(int index, int kind, int nu, int target)
+      : w((int)((unsigned)index | (unsigned)kind << 15 | ((unsigned)nu & 15u) << 17 | (unsigned)target << 21)) {}
+  __host__ __device__ int index() const { return w & 0x7fff; }
+  __host__ __device__ int kind() const { return (w >> 15) & 3; }   // 0: more to come, 1: entry done, 2: partial
+  __host__ __device__ int nu() const { return (int)((unsigned)w << 11) >> 28; }
+  __host__ __device__ int target() const { return (int)((unsigned)w >> 21); }   // row * 33 + column, or the slot
+};
+// a product of two slot values; operand 0: none
+struct PairWord {
+  int w;
+  __host__ __device__ explicit PairWord(int word) : w(word) {}
+  __host__ __device__ PairWord(int a, int b, int operand) : w(a | b << 8 | operand << 16) {}
+  __host__ __device__ int a() const { return w & 0xff; }
+  __host__ __device__ int b() const { return (w >> 8) & 0xff; }
+  __host__ __device__ int operand() const { return w >> 16; }
+};
+
 // Device tables of one network for a group of `lanes` threads integrating one
 // cell: the warp-per-cell integrator (lanes = 32, neq <= 32) and the
 // CTA-per-cell integrator (lanes = 32*ceil(neq/32), at least 64; neq <= 252
@@ -49,15 +91,14 @@ struct WarpTables {
                               //  operand | sign of nu << 31)
   int2 *pairs = nullptr;      // [npairs] slots (a, b) of each reactant pair
   // The warp integrator's term tables in one packed block of `wtab_words` ints,
-  // which a block copies to shared memory (offsets in ints):
-  //   rt   [rhs_len4][32]  kn index << 3 | operand << 18 | sign of nu << 31 | 1 on the last term of a partial sum
-  //   h    [hlen4][32]     which * nreac + reaction | kind << 14 | nu << 16 (signed, 5 bits) | target << 21,
-  //                       target = row * 33 + column of the Newton matrix, or the slot
-  //                       (both padded to whole groups of four with terms that add a zero)
-  //   pk   [pk_len][32]   the pair products in the order rhs() forms them, slot a | slot b << 8 | operand << 16
-  //                       (operand 0: none): rounds 0..4 share their instruction with the levels of the x_e
-  //                       sum (lanes 16 >> round and up are free), the others follow, with every pair of the
-  //                       electron among them
+  // which a block copies to shared memory (offsets in ints; words: TermWord,
+  // JacWord, PairWord above):
+  //   rt   [rhs_len4][32]  the right-hand side's terms
+  //   h    [hlen4][32]     the Jacobian's contributions
+  //                        (both padded to whole groups of four with terms that add a zero)
+  //   pk   [pk_len][32]    the pair products in the order rhs() forms them: rounds 0..4 share their
+  //                        instruction with the levels of the x_e sum (lanes 16 >> round and up are
+  //                        free), the others follow, with every pair of the electron among them
   //   pl   [1+plist_len][32] bytes: first partial slot of each lane, then the partial slots of each species
   //   rab  [nreac] 16-bit: slot a | slot b << 8
   //   bnd  [nbnd]         target | first slot << 11 | last slot + 1 << 19 of the runs across chunks

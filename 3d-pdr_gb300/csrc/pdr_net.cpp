@@ -564,6 +564,7 @@ int build_device_tables(pdr_net *net) {
   // the packed term tables hold a reaction in 16 bits and a slot in 8: larger
   // networks get no integrator tables (the solve entry points reject them)
   if (h.nreac >= 65536 || neq + 2 > 255) return rc;
+  constexpr int UNPACKABLE = 1;   // build(): the packed tables cannot hold the network
   auto build = [&](int G, WarpTables &w, size_t max_merged) -> int {
     w.neq = neq;
     w.nreac = h.nreac;
@@ -783,15 +784,16 @@ int build_device_tables(pdr_net *net) {
       w.nslots = slot;
     }
     // the warp integrator's packed tables (pdr_internal.h); a network beyond
-    // their fields (8,191 rate constants) is left to the block integrator
+    // their fields is left to the block integrator
     std::vector<int> wt;
     if (G == kWarp) {
-      if (nkn >= 8192 || w.nparts >= 127 || w.nop >= 1024 || neq * (kWarp + 1) + kWarp >= 2048 || w.nslots >= 255)
-        return PDR_E_NET;
+      if (nkn > TermWord::MAX_RATE || 2 * h.nreac - 1 > JacWord::MAX_INDEX || w.nparts >= 127 ||
+          w.nop > TermWord::MAX_OPERAND || neq * (kWarp + 1) + kWarp > JacWord::MAX_TARGET || w.nslots >= 255)
+        return UNPACKABLE;
       std::vector<int> free_pairs, el_pairs, pk;
       for (int p = 0; p < (int)pairs.size(); p++)
         (pairs[p].x == neq || pairs[p].y == neq ? el_pairs : free_pairs).push_back(p);
-      auto word = [&](int p) { return pairs[p].x | (pairs[p].y << 8) | ((neq + 2 + p) << 16); };
+      auto word = [&](int p) { return PairWord(pairs[p].x, pairs[p].y, neq + 2 + p).w; };
       pk.assign(5 * kWarp, 0);
       size_t at = 0;
       for (int k = 0; k < 5; k++)
@@ -812,23 +814,20 @@ int build_device_tables(pdr_net *net) {
         plb[l] = (unsigned char)next;
         for (int t = 0; t < w.rhs_len; t++) {
           const int fl = (int)((unsigned)rt[t * kWarp + l].x >> 16);
-          if (fl && fl - 1 != next++) return PDR_E_NET;
+          if (fl && fl - 1 != next++) return UNPACKABLE;
         }
       }
       for (int t = 0; t < w.rhs_len4; t++)
         for (int l = 0; l < kWarp; l++) {
           const int2 e = t < w.rhs_len ? rt[t * kWarp + l] : make_int2(nkn, ONE);
-          wt.push_back((int)((((unsigned)e.x & 0xffffu) << 3) | (((unsigned)e.y & 0x7ffu) << 18) |
-                             ((unsigned)e.y & 0x80000000u) | ((unsigned)e.x >> 16 ? 1u : 0u)));
+          wt.push_back((int)TermWord(e.x & 0xffff, e.y & 0x7fffffff, e.y < 0, ((unsigned)e.x >> 16) != 0u).w);
         }
       w.wt_h = (int)wt.size();
       for (const int2 &t : hxy) {
-        const unsigned r = (unsigned)t.x & 0xffffu, which = ((unsigned)t.x >> 16) & 1u, kind = ((unsigned)t.x >> 17) & 3u;
-        const int nu = t.x >> 19;
-        if (nu < -16 || nu > 15) return PDR_E_NET;
-        const unsigned row = (unsigned)t.y & 0xffu, col = ((unsigned)t.y >> 8) & 0xffu, slot = (unsigned)t.y >> 16;
-        const unsigned target = kind == 2 ? slot : row * (kWarp + 1) + col;
-        wt.push_back((int)((which * (unsigned)h.nreac + r) | (kind << 14) | (((unsigned)nu & 31u) << 16) | (target << 21)));
+        const int r = t.x & 0xffff, which = (t.x >> 16) & 1, kind = (t.x >> 17) & 3, nu = t.x >> 19;
+        if (nu < JacWord::MIN_NU || nu > JacWord::MAX_NU) return UNPACKABLE;
+        const int row = t.y & 0xff, col = (t.y >> 8) & 0xff, slot = (int)((unsigned)t.y >> 16);
+        wt.push_back(JacWord(which * h.nreac + r, kind, nu, kind == 2 ? slot : row * (kWarp + 1) + col).w);
       }
       wt.resize(w.wt_h + (size_t)w.hlen4 * kWarp, 0);
       w.wt_pk = (int)wt.size();
@@ -911,7 +910,7 @@ int build_device_tables(pdr_net *net) {
     // a warp integrator keeps its rate constants in shared memory: at most 96
     // merged groups keep the mixed form at 16 warps per SM
     const int e = build(kWarp, net->warp, 96);
-    if (e) rc = e;
+    if (e && e != UNPACKABLE) rc = e;
     net->warp_ok = (e == 0);
   }
   {
