@@ -98,7 +98,8 @@ struct WarpTables {
   //                        (both padded to whole groups of four with terms that add a zero)
   //   pk   [pk_len][32]    the pair products in the order rhs() forms them: rounds 0..4 share their
   //                        instruction with the levels of the x_e sum (lanes 16 >> round and up are
-  //                        free), the others follow, with every pair of the electron among them
+  //                        free), the others follow, with every pair of the electron among them; at
+  //                        least six rounds, x_e being stored at the start of the sixth
   //   pl   [1+plist_len][32] bytes: first partial slot of each lane, then the partial slots of each species
   //   rab  [nreac] 16-bit: slot a | slot b << 8
   //   bnd  [nbnd]         target | first slot << 11 | last slot + 1 << 19 of the runs across chunks

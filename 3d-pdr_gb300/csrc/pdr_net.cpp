@@ -804,6 +804,8 @@ int build_device_tables(pdr_net *net) {
         if (i % kWarp == 0) pk.resize(pk.size() + kWarp, 0);
         pk[(5 + i / kWarp) * kWarp + i % kWarp] = word(rest[i]);
       }
+      // round 5 is where x_e, summed in the rounds before, gets its slot: it is there for every network
+      if (rest.empty()) pk.resize(6 * kWarp, 0);
       w.pk_len = (int)pk.size() / kWarp;
       w.wt_rt = 0;
       w.rhs_len4 = (w.rhs_len + 3) & ~3;

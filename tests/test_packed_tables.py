@@ -72,3 +72,13 @@ def many(n, seed):
                                         (33000, "block")])
 def test_size_of_the_network(check, tmp_path, nreac, want):
     run(check, *write_network(tmp_path, many(nreac, nreac)), "-", want)
+
+
+def test_electron_alone_in_its_reactions(check, tmp_path):
+    """No pair of the electron and few enough pairs that they all fit beside the
+    x_e sum (129 free lanes): a one-body electron reaction still reads x_e."""
+    pairs = [(NAMES[i], NAMES[j]) for i in range(16) for j in range(i, 16)]
+    for npair in (1, 129, 130):
+        reac = [(p, [NAMES[20 + k % 12]]) for k, p in enumerate(pairs[:npair])] + [(("e-", "FREEZE"), ["N3", "N19"])]
+        out = run(check, *write_network(tmp_path, reac), "-", "warp")
+        assert "pair rounds 6" in out
