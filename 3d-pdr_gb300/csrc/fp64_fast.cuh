@@ -18,13 +18,14 @@
 //  * a small FP32 correction t of an FP64 coefficient c with a known exponent
 //    is added as an integer to c's mantissa (add_rel), not by a conversion and
 //    an FP64 add;
-//  * divisions and reciprocal square roots start from the FP32 unit's value
+//  * divisions, reciprocals and square roots start from the FP32 unit's value
 //    and are finished by FP64 residual steps (Markstein 2000).
 //
 // Against 113-bit references over the ranges the kernels use (3,000,000 points
 // each, on the CPU): exp_fast 0.502 ulp, powk 0.70 ulp, log2k 1.5e-14 of
 // 1024 log2(x) absolute, rsqrt_fast 0.64 ulp; div_fast rounds as the division
-// in every one.
+// in every one, and to 0.5 + 2^-35 ulp by its construction.  rcp_rn and sqrt_rn
+// round as the IEEE operations for every operand.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -40,6 +41,20 @@ constexpr double K_LN2 = 1477.3197218702985;        // 1024/ln 2
 constexpr float K_LN2_LO = 2.08438003e-14f;         //   its rounding error
 constexpr double C1 = 0.00067690154351557157;       // ln 2/1024
 constexpr double C2 = 2.2909784980688164e-07;       // C1^2/2 = 1.9218... 2^-23
+
+#ifdef __CUDACC__   // (a host build of this file brings its own)
+// the FP32 unit's approximations, to about an ulp
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+#endif
 
 __device__ __forceinline__ int hi32(double x) { return __double2hiint(x); }
 __device__ __forceinline__ int lo32(double x) { return __double2loint(x); }
@@ -166,8 +181,7 @@ __device__ __forceinline__ double rcp_seed(double b) {
   // the mantissa as bh + bl, 24 + 24 bits
   const float bh = __uint_as_float((__funnelshift_l(l, h, 3) & 0x7fffffu) | 0x3f800000u);
   const float bl = (float)((l & 0x1fffffffu) >> 5) * 7.105427357601002e-15f;   // 2^-47
-  float y0;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(bh));
+  float y0 = rcp_approx(bh);
   y0 = fminf(fmaxf(y0, 0.5f), 0.99999994f);        // 1/b is in (1/2, 1]
   const float e = fmaf(-bl, y0, fmaf(-bh, y0, 1.0f));
   const float y1 = fmaf(y0 * e, e, y0 * e);
@@ -178,14 +192,28 @@ __device__ __forceinline__ double rcp_seed(double b) {
   bits += (long long)__float2int_rn(y1 * 2251799813685248.0f) << 2;             // 2^51
   return __longlong_as_double(bits | (long long)((unsigned long long)(h & 0x80000000u) << 32));
 }
-// 1/b, rounded (2 FP64 instructions where the operand and result are normal)
+// q, within 2^-35 ulp of the rounded result, or the neighbour that is nearer to
+// the exact one: res is the exact residual of q, whose magnitude passes `half`
+// (the bits of a positive value) where the exact result lies half an ulp beyond
+// q.  Below a power of two the ulp is half as large.  Integer operations only.
+__device__ __forceinline__ double settle(double q, double res, long long half) {
+  const long long r = __double_as_longlong(res), mag = r & 0x7fffffffffffffffll, qb = __double_as_longlong(q);
+  const long long below = half - ((qb & 0xfffffffffffffll) ? 0ll : 1ll << 52);
+  return __longlong_as_double(qb + (r >= 0 ? (mag > half ? 1 : 0) : (mag >= below ? -1 : 0)));
+}
+// 1/b, rounded (3 FP64 instructions where the operand and result are normal).
+// The second-order term that the first two leave out is 2^-88 of the result,
+// enough to round the wrong way beside the midpoint of two doubles; the residual
+// 1 - b q, an exact FMA, is b ulp(q)/2 at that midpoint.
 __device__ __forceinline__ double rcp_rn(double b) {
   const unsigned e = ((unsigned)hi32(b) >> 20) & 0x7ff;
   if (e - 2u >= 2042u) return __drcp_rn(b);   // zero, denormal, infinite, NaN, or a denormal result
-  const double y = rcp_seed(b);
-  return fma(y, fma(-b, y, 1.0), y);
+  const double y = rcp_seed(b), q = fma(y, fma(-b, y, 1.0), y);
+  const long long eq = (long long)(((unsigned)hi32(q) >> 20) & 0x7ff) - 1023;
+  return settle(q, fma(-b, q, 1.0), (__double_as_longlong(b) & 0x7fffffffffffffffll) + (eq - 53) * (1ll << 52));
 }
-// a/b for normal operands and result
+// a/b for normal operands and result: within 0.5 + 2^-35 ulp (the terms left out
+// are 2^-88 of the quotient, so one in about 2^35 may round the other way)
 __device__ __forceinline__ double div_fast(double a, double b) {
   const double y = rcp_seed(b);
   const double q = a * y;
@@ -197,20 +225,22 @@ __device__ __forceinline__ double div_any(double a, double b) {
   if (ea - 64u > 1918u || eb - 64u > 1918u || ea - eb + 959u > 1918u) return a / b;
   return div_fast(a, b);
 }
-// sqrt(x), rounded: six FP64 instructions where x is within FP32's normal range
+// sqrt(x), rounded: seven FP64 instructions where x is within FP32's normal range
+// (six leave out 2^-88 of the root; the exact residual x - g^2 settles the rest:
+// at the midpoint above g it is g ulp(g) + ulp(g)^2/4, in whole ulp(g)^2 beyond it)
 __device__ __forceinline__ double sqrt_rn(double x) {
   if ((unsigned)hi32(x) - 0x38200000u > 0x0f000000u) return __dsqrt_rn(x);   // zero, negative, tiny, huge, NaN
-  float y0;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d2f(x)));
+  const float y0 = rsqrt_approx(d2f(x));
   const double y = f2d(y0), g = x * y, h = scale2(y, -1);
   const double r = fma(-g, h, 0.5);              // (1 - x y^2)/2
   const double g1 = fma(g, r, g), h1 = fma(h, r, h);
-  return fma(fma(-g1, g1, x), h1, g1);
+  const double g2 = fma(fma(-g1, g1, x), h1, g1);
+  const long long eg = (long long)((unsigned)hi32(g2) >> 20) - 1023;
+  return settle(g2, fma(-g2, g2, x), __double_as_longlong(g2) + (eg - 52) * (1ll << 52));
 }
 // 1/sqrt(x), x positive normal within FP32's range
 __device__ __forceinline__ double rsqrt_fast(double x) {
-  float y0;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d2f(x)));
+  const float y0 = rsqrt_approx(d2f(x));
   const double y = f2d(y0 * 0.9999996f);            // from below, so that e > 0
   const double e = fma(-(x * y), y, 1.0);
   // y (1 + e/2 + 3 e^2/8), e < 2^-18
