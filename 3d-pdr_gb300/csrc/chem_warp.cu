@@ -179,7 +179,7 @@ __device__ __forceinline__ bool lu_rows(MT *a, int ld, int lane, int &mystep, MT
 #pragma unroll
       for (int j = t; j < 4; j++) u[j] = bcast(r[j], p);
       MT rinv;
-      if constexpr (sizeof(MT) == 8) rinv = fp64::rcp_rn(u[t]);
+      if constexpr (sizeof(MT) == 8) rinv = fp64::rcp_near(u[t]);
       else rinv = __frcp_rn(u[t]);
       if (lane == p) { mystep = k0 + t; invd = rinv; perm[k0 + t] = p; }
       if (mystep < 0) {

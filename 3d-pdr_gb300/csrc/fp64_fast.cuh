@@ -24,8 +24,8 @@
 // Against 113-bit references over the ranges the kernels use (3,000,000 points
 // each, on the CPU): exp_fast 0.502 ulp, powk 0.70 ulp, log2k 1.5e-14 of
 // 1024 log2(x) absolute, rsqrt_fast 0.64 ulp; div_fast rounds as the division
-// in every one, and to 0.5 + 2^-35 ulp by its construction.  rcp_rn and sqrt_rn
-// round as the IEEE operations for every operand.
+// in every one, and to 0.5 + 2^-35 ulp by its construction, as rcp_near.  sqrt_rn
+// rounds as the IEEE square root for every operand.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -192,28 +192,17 @@ __device__ __forceinline__ double rcp_seed(double b) {
   bits += (long long)__float2int_rn(y1 * 2251799813685248.0f) << 2;             // 2^51
   return __longlong_as_double(bits | (long long)((unsigned long long)(h & 0x80000000u) << 32));
 }
-// q, within 2^-35 ulp of the rounded result, or the neighbour that is nearer to
-// the exact one: res is the exact residual of q, whose magnitude passes `half`
-// (the bits of a positive value) where the exact result lies half an ulp beyond
-// q.  Below a power of two the ulp is half as large.  Integer operations only.
-__device__ __forceinline__ double settle(double q, double res, long long half) {
-  const long long r = __double_as_longlong(res), mag = r & 0x7fffffffffffffffll, qb = __double_as_longlong(q);
-  const long long below = half - ((qb & 0xfffffffffffffll) ? 0ll : 1ll << 52);
-  return __longlong_as_double(qb + (r >= 0 ? (mag > half ? 1 : 0) : (mag >= below ? -1 : 0)));
-}
-// 1/b, rounded (3 FP64 instructions where the operand and result are normal).
-// The second-order term that the first two leave out is 2^-88 of the result,
-// enough to round the wrong way beside the midpoint of two doubles; the residual
-// 1 - b q, an exact FMA, is b ulp(q)/2 at that midpoint.
-__device__ __forceinline__ double rcp_rn(double b) {
+// 1/b within 0.5 + 2^-35 ulp (2 FP64 instructions where the operand and result
+// are normal; the terms left out are 2^-88 of the result, so one in about 2^35
+// rounds the other way.  Settled like the square root below it cost 20,011 CO
+// cells 5 %, 3.10 -> 3.25 ms, and 1,500 cells of FP64 chemistry 2 %.)
+__device__ __forceinline__ double rcp_near(double b) {
   const unsigned e = ((unsigned)hi32(b) >> 20) & 0x7ff;
   if (e - 2u >= 2042u) return __drcp_rn(b);   // zero, denormal, infinite, NaN, or a denormal result
-  const double y = rcp_seed(b), q = fma(y, fma(-b, y, 1.0), y);
-  const long long eq = (long long)(((unsigned)hi32(q) >> 20) & 0x7ff) - 1023;
-  return settle(q, fma(-b, q, 1.0), (__double_as_longlong(b) & 0x7fffffffffffffffll) + (eq - 53) * (1ll << 52));
+  const double y = rcp_seed(b);
+  return fma(y, fma(-b, y, 1.0), y);
 }
-// a/b for normal operands and result: within 0.5 + 2^-35 ulp (the terms left out
-// are 2^-88 of the quotient, so one in about 2^35 may round the other way)
+// a/b for normal operands and result: within 0.5 + 2^-35 ulp, as rcp_near
 __device__ __forceinline__ double div_fast(double a, double b) {
   const double y = rcp_seed(b);
   const double q = a * y;
@@ -224,6 +213,15 @@ __device__ __forceinline__ double div_any(double a, double b) {
   const unsigned ea = ((unsigned)hi32(a) >> 20) & 0x7ff, eb = ((unsigned)hi32(b) >> 20) & 0x7ff;
   if (ea - 64u > 1918u || eb - 64u > 1918u || ea - eb + 959u > 1918u) return a / b;
   return div_fast(a, b);
+}
+// q, within 2^-35 ulp of the rounded result, or the neighbour that is nearer to
+// the exact one: res is the exact residual of q, whose magnitude passes `half`
+// (the bits of a positive value) where the exact result lies half an ulp beyond
+// q.  Below a power of two the ulp is half as large.  Integer operations only.
+__device__ __forceinline__ double settle(double q, double res, long long half) {
+  const long long r = __double_as_longlong(res), mag = r & 0x7fffffffffffffffll, qb = __double_as_longlong(q);
+  const long long below = half - ((qb & 0xfffffffffffffll) ? 0ll : 1ll << 52);
+  return __longlong_as_double(qb + (r >= 0 ? (mag > half ? 1 : 0) : (mag >= below ? -1 : 0)));
 }
 // sqrt(x), rounded: seven FP64 instructions where x is within FP32's normal range
 // (six leave out 2^-88 of the root; the exact residual x - g^2 settles the rest:

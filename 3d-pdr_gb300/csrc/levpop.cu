@@ -231,7 +231,7 @@ __device__ __forceinline__ bool gauss_full(double *a, double *b, int n, double *
     }
     const double piv = a[icol * n + icol];
     if (piv == 0.0) { ok = false; break; }
-    const double pivinv = fp64::rcp_rn(piv);
+    const double pivinv = fp64::rcp_near(piv);
     if (lane == 0) x[icol] = pivinv;
     for (int p = lane; p < nact; p += 32) l[p] = a[act[p] * n + icol] * pivinv;
     __syncwarp();

@@ -1,10 +1,12 @@
 // Host checks of fp64_fast.cuh, compiled with the intrinsics of cuda_runtime.h
 // beside this file.
-//  rounding  rcp_rn and sqrt_rn round as the IEEE operations, whatever the FP32
-//            unit's start value (moved by up to 2 ulp) -- on random operands and on
-//            those whose results lie nearest to the midpoint of two doubles
+//  rounding  sqrt_rn rounds as the IEEE operation and rcp_near is within 0.5 + 2^-35 ulp,
+//            whatever the FP32 unit's start value (moved by up to 2 ulp) -- on random operands
+//            and on those whose results lie nearest to the midpoint of two doubles
 // Usage: fp64_check rounding; exit 0 when every check holds.
 #include "../../3d-pdr_gb300/csrc/fp64_fast.cuh"
+
+#include <quadmath.h>
 
 #include <cstdio>
 #include <random>
@@ -48,6 +50,15 @@ static int check_rounding() {
     if (__double_as_longlong(got) == __double_as_longlong(want)) return;
     if (bad++ < 10) std::printf("%s(%.17g) with the start value %+d ulp: %.17g, not %.17g\n", what, x, g_seed_ulps, got, want);
   };
+  // the nearest double, or the other neighbour where the exact value is within 2^-35 ulp of their midpoint
+  auto near_rcp = [&](double x, double got) {
+    n++;
+    if (__double_as_longlong(got) == __double_as_longlong(1.0 / x)) return;
+    // in ulps of the result (distances from a midpoint are exact to 2^-60 ulp in 113 bits)
+    const __float128 off = fabsq((1 / (__float128)x - got) / std::ldexp(1.0, std::ilogb(1.0 / x) - 52)) - 0.5Q;
+    if (fabsq(off) <= ldexpq(1.0Q, -35)) return;
+    if (bad++ < 10) std::printf("rcp_near(%.17g) with the start value %+d ulp: %.17g\n", x, g_seed_ulps, got);
+  };
   std::vector<double> sq = hard_squares(), rc;
   std::printf("%zu hard square roots\n", sq.size());
   if (sq.size() < 1000) bad++;
@@ -71,7 +82,7 @@ static int check_rounding() {
   }
   for (g_seed_ulps = -2; g_seed_ulps <= 2; g_seed_ulps++) {
     if (g_seed_ulps != -2 && g_seed_ulps != 2)
-      for (double x : rc) same("rcp_rn", x, rcp_rn(x), 1.0 / x);
+      for (double x : rc) near_rcp(x, rcp_near(x));
     for (double x : sq) same("sqrt_rn", x, sqrt_rn(x), std::sqrt(x));
   }
   std::printf("%ld of %ld misrounded\n", bad, n);
