@@ -182,7 +182,7 @@ struct RateTables {
   int *dup = nullptr;         // DUPLICATE
   int *dup_next = nullptr;    // DUPLICATE(I+1) or -1 past the end
   double *alpha = nullptr, *beta = nullptr, *gamma = nullptr, *rtmin = nullptr, *rtmax = nullptr;
-  int *flags = nullptr;       // bit0: reactant-1 name starts with 'G'; bit1: H2 photo sets NRH2;
+  int *flags = nullptr;       // bit0: reactant-1 name starts with 'G'; bit1: no rate below RTMIN (thermal, gamma < -200)
                               // bit2: HD photo sets NRHD
   // evaluation order: the reactions whose rate is a sum over the rays (the
   // photo-reactions and photodesorption), grouped by kind, then the others,

@@ -489,6 +489,7 @@ int build_device_tables(pdr_net *net) {
     for (int i = 0; i < h.nreac; i++) {
       dn[i] = (i + 1 < h.nreac) ? h.dup[i + 1] : -1;
       if (!h.reac[i][0].empty() && h.reac[i][0][0] == 'G') flags[i] |= 1;
+      if (h.rate_kind[i] == RK_THERMAL && h.gamma[i] < -200.0) flags[i] |= 2;
     }
     net->rates.nreac = h.nreac;
     net->rates.kind = upload(net, kind, rc);

@@ -471,21 +471,41 @@ struct RayRates {
   double av2, rs, h2, hd, co, ci;
 };
 
+// The reference's expressions jump where they change (SCATTER by 3.8e-4 at tau =
+// 1), and the fast path's arguments may be an ulp or so from the reference's.  So
+// each choice is made on all the bits of the argument, by integer compares, and
+// within 4,096 ulp (9e-13) of a jump the reference's own expression decides: a
+// rare call.
+__device__ __forceinline__ bool at_jump(double x, double jump) {
+  return (unsigned long long)(__double_as_longlong(x) - __double_as_longlong(jump) + 4096) < 8192ull;
+}
+__device__ __noinline__ double scatter_at_jump(double av, double nco, double nh2, bool co, int linear) {
+  return scatter(av, co ? lbar(nco, nh2) : 1000.0, linear);
+}
+__device__ __noinline__ double h2_taud(double nh2, double v_turb) {
+  const double dopw = v_turb / (1000.0 * 1.0e-8);
+  return nh2 * 0.5 * (1.497358985e-2) * 1.0e-2 / dopw;
+}
+
 // SCATTER(A_V, lambda) (shield.F90:449) from tl = tau(lambda) 1024/ln 2: one
 // exponential below tau = 1, else five, those with an exponent of 100 or more
-// left out
+// left out (c_scat_end: where that is, and tau = 1 in the first place); jump: the
+// caller has to take the reference's expression
 __constant__ double c_scat_a[6] = {1.000, 2.006, -1.438, 0.7364, -0.5076, -0.0592};
 __constant__ double c_scat_k[6] = {0.7514, 0.8490, 1.013, 1.282, 2.005, 5.832};
 __constant__ float c_scat_kf[6] = {0.7514f, 0.8490f, 1.013f, 1.282f, 2.005f, 5.832f};
-__device__ __forceinline__ double scatter_fast(double tl) {
+__constant__ double c_scat_end[6] = {fp64::K_LN2, 100.0 / 0.8490 * fp64::K_LN2, 100.0 / 1.013 * fp64::K_LN2,
+                                     100.0 / 1.282 * fp64::K_LN2, 100.0 / 2.005 * fp64::K_LN2, 100.0 / 5.832 * fp64::K_LN2};
+__device__ __forceinline__ double scatter_fast(double tl, bool &jump) {
   const float tf = fp64::d2f(tl);
-  const bool thin = tf < (float)fp64::K_LN2;
+  const bool thin = __double_as_longlong(tl) < __double_as_longlong(fp64::K_LN2);
+  jump = at_jump(tl, fp64::K_LN2);
   double s = 0.0;
   for (int i = thin ? 0 : 1; i < (thin ? 1 : 6); i++) {
-    const float arg = c_scat_kf[i] * tf;
-    if (arg >= 147731.97f) continue;   // an exponent of 100 or more
+    jump |= at_jump(tl, c_scat_end[i]);
+    if (__double_as_longlong(tl) >= __double_as_longlong(c_scat_end[i])) continue;
     float kf;
-    const int k = fp64::rint_f(-arg, kf);
+    const int k = fp64::rint_f(-c_scat_kf[i] * tf, kf);
     const double r = fma(-c_scat_k[i], tl, fp64::flip(fp64::f2d(kf)));
     const double t = c_scat_a[i] * fp64::exp2_int(k);
     s = fma(t, fma(r, fp64::exp2_slope(r), 1.0), s);
@@ -494,8 +514,9 @@ __device__ __forceinline__ double scatter_fast(double tl) {
 }
 
 // H2SHIELD1 (shield.F90:231) for a positive Doppler width
-__device__ __forceinline__ double h2shield_fast(double nh2, const RateShield &S) {
-  const double taud = nh2 * S.taud;
+__device__ __forceinline__ double h2shield_fast(double nh2, const RateShield &S, double v_turb) {
+  double taud = nh2 * S.taud;
+  if (at_jump(taud, 2.0) || at_jump(taud, 10.0) || at_jump(taud, 100.0)) taud = h2_taud(nh2, v_turb);
   double jd = 1.0;
   if (taud >= 2.0) {
     const double p = taud < 10.0 ? -1.25 : (taud < 100.0 ? -1.15 : -1.0667);
@@ -630,15 +651,21 @@ __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_co
         }
         R.av2 = av * fp64::K_LN2;
         if (S.has_h2 | S.has_hd) {
-          const double s = R.rs * scatter_fast(R.av2 * S.x1000[linear]);
-          if (S.has_h2) R.h2 = s * h2shield_fast(nh2, S);
-          if (S.has_hd) R.hd = s * h2shield_fast(nhd, S);
+          bool jump;
+          double s = scatter_fast(R.av2 * S.x1000[linear], jump);
+          if (jump) s = scatter_at_jump(av, 0.0, 0.0, false, linear);
+          s = R.rs * s;
+          if (S.has_h2) R.h2 = s * h2shield_fast(nh2, S, A.ph.v_turb);
+          if (S.has_hd) R.hd = s * h2shield_fast(nhd, S, A.ph.v_turb);
         }
         if (S.has_co) {
           constexpr double LG = 0.00029397460514060664;   // log10(2)/1024
           const double u = fp64::log2k1(nco + 1.0) * LG, w = fp64::log2k1(nh2 + 1.0) * LG;
           const double tl = R.av2 * (xlambda_lbar(u, w, linear) * (1.0 / 1.086));
-          R.co = R.rs * scatter_fast(tl) * coshield_fast(u, w);
+          bool jump;
+          double s = scatter_fast(tl, jump);
+          if (jump) s = scatter_at_jump(av, nco, nh2, true, linear);
+          R.co = R.rs * s * coshield_fast(u, w);
         }
         // the C photo-rate's H2 line opacity without its T^0.27, which the cell's lane may still be computing
         if (S.has_ci) R.ci = nh2 > 0.0 ? fp64::powk(fp64::log2k(nh2 * (1.0 / 1.59e21)), 0.45) : 0.0;
@@ -726,7 +753,7 @@ __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_co
               m -= fp64::rint_f(fminf(fmaxf(arg, -3.0e6f), 3.0e6f), kf);
               const double y = fma(g, C.Gl, fma(g, C.Gh, fp64::flip(fp64::f2d(kf))));
               x = (cls == RC_BOTH) ? x - y : fp64::flip(y);
-              if (gf < -200.0f) zero = C.t < __ldg(&T.rtmin[r]);
+              if (flags & 2) zero = C.t < __ldg(&T.rtmin[r]);
             }
             if (cls == RC_CRPHOT) a = a * C.zeta;
             k = zero ? 0.0 : scaled_exp2(a, m, far ? 0.0 : x);
