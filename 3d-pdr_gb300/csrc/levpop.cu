@@ -276,11 +276,12 @@ __device__ __forceinline__ bool gauss_full(double *a, double *b, int n, double *
 // refinement step would make to population x: above 1e-6 of the coolant
 // density it must be below 1e-7 of x, above 1e-12 of the density below 1e-4
 // of x (ten times inside the 1e-6 and 1e-3 the results are held to), and it
-// must contract (at most half the previous correction, or negligible)
+// must contract (at most half the previous correction, or negligible).  A NaN
+// among them is refused; as itself is a finite FP32 value.
 __device__ __forceinline__ bool refine_ok(double ax, double as, double prev, double dens) {
   const bool contracts = as <= 0.5 * prev || as <= 1.0e-12 * ax;
-  if (ax > 1.0e-6 * dens) return as <= 1.0e-7 * ax && contracts;
-  if (ax > 1.0e-12 * dens) return as <= 1.0e-4 * ax && contracts;
+  if (!(ax <= 1.0e-6 * dens)) return as <= 1.0e-7 * ax && contracts;
+  if (!(ax <= 1.0e-12 * dens)) return as <= 1.0e-4 * ax && contracts;
   return true;
 }
 
@@ -613,18 +614,25 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
       // 1 / row maximum), its LU factors, then x = inv(DM) D b and up to two
       // refinement steps x += inv(DM) D (b - M x) with the residual in FP64
       // and the correction in FP32.  Each step is accepted by the size of the
-      // correction the next would make (refine_ok); otherwise the cell is
-      // re-solved by the FP64 elimination (R is intact).
+      // correction the next would make (refine_ok); otherwise, and where the
+      // matrix has entries that FP32 cannot hold (2^127 and beyond, NaN), the
+      // cell is re-solved by the FP64 elimination (R is intact).
       float *Mf = reinterpret_cast<float *>(base + L.Mf);
       const int n4 = (n + 3) & ~3, ld = n4 | 1;
       float *upan = reinterpret_cast<float *>(base + L.upan), *dinv = upan + 4 * n4;
       int *perm = reinterpret_cast<int *>(dinv + n4);
       // rows as columns of R^T would be: lane i scales rows i and i + 32
       float s0 = 1.0f, s1 = 1.0f;
+      bool fits = true;
       for (int i = lane; i < n4; i += 32) {
         float mx = 0.0f;
         for (int l = 0; l < n4; l++) {
-          const float v = (i < n && l < n) ? fp64::d2f(R[i * n + l]) : (i == l ? 1.0f : 0.0f);
+          float v = i == l ? 1.0f : 0.0f;
+          if (i < n && l < n) {
+            const double r = R[i * n + l];
+            v = fp64::d2f(r);
+            fits &= (fp64::hi32(r) & 0x7fffffff) < 0x47e00000;   // 2^127
+          }
           Mf[i * ld + l] = v;
           mx = fmaxf(mx, fabsf(v));
         }
@@ -634,37 +642,40 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
         else s1 = sc;
       }
       __syncwarp();
-      ok = lu_pp(Mf, n4, ld, upan, perm, dinv);
-      // b is zero but for its last entry
-      float c0 = lane == n - 1 ? s0 : 0.0f, c1 = lane + 32 == n - 1 ? s1 : 0.0f;
-      lu_pp_solve(Mf, n4, ld, perm, dinv, c0, c1);
-      const double bl = b[n - 1];
-      if (lane < n) x[lane] = (double)c0 * bl;
-      if (lane + 32 < n) x[lane + 32] = (double)c1 * bl;
-      float prev0 = 0.0f, prev1 = 0.0f;
+      ok = __all_sync(FULL, fits);
       bool good = false;
-      for (int it = 0; it < 3 && ok && !good; it++) {
-        __syncwarp();
-        double d0 = lane < n ? b[lane] : 0.0, d1 = lane + 32 < n ? b[lane + 32] : 0.0;
-        row_sums(n, [&](int i, int l, double v) { return fma(-R[i * n + l], x[l], v); }, d0, d1);
-        __syncwarp();
-        c0 = lane < n ? (float)d0 * s0 : 0.0f;
-        c1 = lane + 32 < n ? (float)d1 * s1 : 0.0f;
+      if (ok) {
+        ok = lu_pp(Mf, n4, ld, upan, perm, dinv);
+        // b is zero but for its last entry
+        float c0 = lane == n - 1 ? s0 : 0.0f, c1 = lane + 32 == n - 1 ? s1 : 0.0f;
         lu_pp_solve(Mf, n4, ld, perm, dinv, c0, c1);
-        bool bad = false;
-        auto step = [&](int i, float c, float &prev) {
-          const double sd = (double)c;
-          // from the second correction on, the correction is also the test of
-          // the previous one
-          if (it > 0 && !refine_ok(fabs(x[i]), fabs(sd), (double)prev, dens)) bad = true;
-          if (it < 2) {
-            x[i] += sd;
-            prev = fabsf(c);
-          }
-        };
-        if (lane < n) step(lane, c0, prev0);
-        if (lane + 32 < n) step(lane + 32, c1, prev1);
-        good = (it > 0) && !__any_sync(FULL, bad);
+        const double bl = b[n - 1];
+        if (lane < n) x[lane] = (double)c0 * bl;
+        if (lane + 32 < n) x[lane + 32] = (double)c1 * bl;
+        float prev0 = 0.0f, prev1 = 0.0f;
+        for (int it = 0; it < 3 && ok && !good; it++) {
+          __syncwarp();
+          double d0 = lane < n ? b[lane] : 0.0, d1 = lane + 32 < n ? b[lane + 32] : 0.0;
+          row_sums(n, [&](int i, int l, double v) { return fma(-R[i * n + l], x[l], v); }, d0, d1);
+          __syncwarp();
+          c0 = lane < n ? (float)d0 * s0 : 0.0f;
+          c1 = lane + 32 < n ? (float)d1 * s1 : 0.0f;
+          lu_pp_solve(Mf, n4, ld, perm, dinv, c0, c1);
+          bool bad = false;
+          auto step = [&](int i, float c, float &prev) {
+            const double sd = (double)c;
+            // from the second correction on, the correction is also the test of
+            // the previous one
+            if (it > 0 && (!(fabsf(c) < INFINITY) || !refine_ok(fabs(x[i]), fabs(sd), (double)prev, dens))) bad = true;
+            if (it < 2) {
+              x[i] += sd;
+              prev = fabsf(c);
+            }
+          };
+          if (lane < n) step(lane, c0, prev0);
+          if (lane + 32 < n) step(lane + 32, c1, prev1);
+          good = (it > 0) && !__any_sync(FULL, bad);
+        }
       }
       if (!ok || !good) {
         __syncwarp();
