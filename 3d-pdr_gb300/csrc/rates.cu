@@ -465,10 +465,11 @@ struct CellRates {
   int ok;             // 0: general path
   int neg;            // lowest negative reaction number
 };
-// per-(cell, ray) values: A_V 1024/ln 2, the field, and the field times the
-// shielding functions of H2, HD, CO and C
+// per-(cell, ray) values: A_V 1024/ln 2 = av2 + av2_lo, the field, and the field
+// times the shielding functions of H2, HD, CO and C
 struct RayRates {
   double av2, rs, h2, hd, co, ci;
+  float av2_lo;
 };
 
 // The reference's expressions jump where they change (SCATTER by 3.8e-4 at tau =
@@ -596,10 +597,12 @@ constexpr int RATES_THREADS = 256;
 // a (T/300)^b is 6.7e-17 off (rms, as with a correctly rounded pow) and
 // a exp(-g/T) 6.7e-17 (1.3e-15 where g/T is rounded first).
 // Over all thermal and photo-reactions of 400 full-network cells: thermal
-// 6.0e-17 rms (library functions 6.8e-16), photo 1.64e-16 rms, 1.1e-15 at most
-// (1.58e-16, 1.6e-15), most of it the rounding of gamma A_V in both.  The
-// table's tail in the photo sum would cost an addition and gains nothing (the
-// sum then rounds twice a ray: 1.93e-16, 1.26 -> 1.32 ms).
+// 5.8e-17 rms (library functions 6.8e-16), photo 1.44e-16 rms, 6.8e-16 at most.
+// The reference rounds gamma A_V, and with the library's exp has 1.59e-16 and
+// 1.6e-15 (host evaluation); rounding A_V 1024/ln 2 alone was 1.76e-16, so its
+// low part goes along (no FP64 instruction more).  The table's tail in the
+// photo sum would cost an addition and gains nothing (the sum then rounds twice
+// a ray: 1.93e-16, 1.26 -> 1.32 ms).
 __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_constant__ RatesArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   CellRates *cells = reinterpret_cast<CellRates *>(smem);
@@ -650,6 +653,7 @@ __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_co
           continue;
         }
         R.av2 = av * fp64::K_LN2;
+        R.av2_lo = fp64::d2f(fma(av, fp64::K_LN2, -R.av2)) + fp64::d2f(av) * fp64::K_LN2_LO;
         if (S.has_h2 | S.has_hd) {
           bool jump;
           double s = scatter_fast(R.av2 * S.x1000[linear], jump);
@@ -706,6 +710,9 @@ __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_co
               gf = 1.8f;
               a = 1.7e8 * 2.4e-22 * (C.t < 50.0 ? 3.5e-3 : (C.t < 85.0 ? 4.0e-3 : (C.t < 100.0 ? 5.5e-3 : 7.5e-3)));
             }
+            // the exponent's low part, -g av2_lo ln 2/1024, is a few units of 2^-53:
+            // it goes into the series' leading 1 by an integer addition
+            const float glo = gf * (float)(-fp64::C1 * 9007199254740992.0);
 #pragma unroll 2
             for (int q = 0; q < nrays; q++) {
               const double av2 = R[q].av2;
@@ -713,7 +720,9 @@ __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_co
               const int m = fp64::rint_f(fmaxf(-gf * fp64::d2f(av2), -2.0e6f), kf);
               const double x = fma(-g, av2, fp64::flip(fp64::f2d(kf)));
               const double t = m < -1000 * 1024 ? 0.0 : R[q].rs * fp64::exp2_int(m);
-              k = fma(t, m < -1000 * 1024 ? 1.0 : fma(x, fp64::exp2_slope(x), 1.0), k);
+              const int lo = __float2int_rn(glo * R[q].av2_lo);
+              const double one = __longlong_as_double(0x3ff0000000000000ll + (lo > 0 ? (lo + 1) >> 1 : lo));
+              k = fma(t, m < -1000 * 1024 ? 1.0 : fma(x, fp64::exp2_slope(x), one), k);
             }
           }
         }
