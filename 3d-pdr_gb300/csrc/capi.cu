@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "launch_shape.h"
 #include "pdr_internal.h"
 
 extern "C" {
@@ -451,6 +452,9 @@ int pdr_chem_autotune(const pdr_net *net, int ncell_sample, const double *d_abun
     set_error("pdr_chem_autotune: invalid argument");
     return PDR_E_ARG;
   }
+  int dev = 0, sms = 0;
+  int rc = current_device(&dev, &sms);
+  if (rc) return rc;
   const int ns = net->host.nspec;
   cudaStream_t st = (cudaStream_t)stream;
   double *ab = nullptr;
@@ -462,22 +466,16 @@ int pdr_chem_autotune(const pdr_net *net, int ncell_sample, const double *d_abun
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
-  struct Cand { int wpb, reg, refill; };
-  const Cand warp_cands[] = {{4, 0, 0}, {2, 0, 0}, {4, 1, 0}, {8, 1, 0}, {4, 2, 0}, {2, 2, 0},
-                             {4, 3, 0}, {4, 1, 1}};
-  const Cand cta_cands[] = {{0, 0, 0}, {0, 0, 1}};   // block integrator: work queue or static refill
-  const bool warp_path = (opts->integrator == 1) || (opts->integrator == 0 && net->warp_ok && net->host.neq == 32);
-  const Cand *cands = warp_path ? warp_cands : cta_cands;
-  const int ncand = warp_path ? 8 : 2;
+  // block integrator: work queue or static refill
+  const std::vector<WarpCandidate> cands = uses_warp_path(net, *opts) ? warp_candidates(ncell_sample, eff_sms(*opts, sms))
+                                                                      : std::vector<WarpCandidate>{{0, 0, 0}, {0, 0, 1}};
   const bool log = getenv("PDR_AUTOTUNE_LOG") != nullptr;
   float best = 1e30f;
   pdr_chem_opts best_o = *opts;
-  int rc = 0;
-  for (int ci = 0; ci < ncand; ci++) {
-    const Cand &c = cands[ci];
+  for (const WarpCandidate &c : cands) {
     pdr_chem_opts o = *opts;
-    o.warps_per_block = c.wpb;
-    o.reg_variant = c.reg;
+    o.warps_per_block = c.warps_per_block;
+    o.reg_variant = c.reg_variant;
     o.refill = c.refill;
     o.blocks_per_sm = 0;
     // the best of two timed runs: the first of a shape also pays its
@@ -498,8 +496,8 @@ int pdr_chem_autotune(const pdr_net *net, int ncell_sample, const double *d_abun
     }
     if (rc) break;
     if (log)
-      fprintf(stderr, "pdr_chem_autotune: warps_per_block %d reg_variant %d refill %d: %.3f ms\n", c.wpb, c.reg,
-              c.refill, ms);
+      fprintf(stderr, "pdr_chem_autotune: warps_per_block %d reg_variant %d refill %d: %.3f ms\n",
+              c.warps_per_block, c.reg_variant, c.refill, ms);
     if (ms < best) { best = ms; best_o = o; }
   }
   cudaEventDestroy(t0);

@@ -35,6 +35,7 @@
 
 #include "bdf_core.cuh"
 #include "fp64_fast.cuh"
+#include "launch_shape.h"
 #include "pdr_internal.h"
 
 namespace pdr {
@@ -813,11 +814,7 @@ int launch_chem_warp(const pdr_net *net, int ncell, double *ab, const double *ra
   // all cells; the FP64 pass over a device-side list keeps the work queue
   const bool one_per_cell = (o.refill == 2) && !cell_list;
   A.refill_static = (o.refill == 1 || one_per_cell) ? 1 : 0;
-  // defaults, the fastest shapes measured on GB300: mixed 128 registers with
-  // 8-warp blocks (16 warps/SM), FP64 168 registers with one 12-warp block per
-  // SM, so that its warps share one copy of the term tables
-  const int rv = (o.reg_variant >= 0 && o.reg_variant <= 3) ? o.reg_variant : (mixed ? 1 : 2);
-  if (rv >= 2 && o.warps_per_block > 4) return PDR_E_ARG;   // the caller's blocks take at most 4 warps there
+  const int rv = warp_variant(o, mixed);
   const bool zsh = (rv == 1 || rv == 3);
   const size_t per_warp = chem_warp_smem_per_warp(T, mixed, zsh), tables = 4 * (size_t)T.wtab_words;
   int dev = 0, optin = 0;
@@ -825,9 +822,8 @@ int launch_chem_warp(const pdr_net *net, int ncell, double *ab, const double *ra
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   dev &= 63;
-  int wpb = o.warps_per_block > 0 ? o.warps_per_block : ((rv >= 2) ? 12 : 8);
-  if (o.warps_per_block <= 0 && rv >= 2 && per_warp * 12 + tables + 1024 > (size_t)optin) wpb = 4;   // a larger network
-  if (wpb > 12 || (wpb > 8 && rv < 2)) return PDR_E_ARG;
+  const int wpb = warp_block(o, rv, per_warp, tables, (size_t)optin);
+  if (wpb < 1) return PDR_E_ARG;
   const int variant = (mixed ? 4 : 0) + rv;
   using KFn = void (*)(ChemArgs, int, const int *);
   static const KFn kernels[8] = {chem_warp_kernel<32, false, 0>, chem_warp_kernel<32, false, 1>,
@@ -842,8 +838,8 @@ int launch_chem_warp(const pdr_net *net, int ncell, double *ab, const double *ra
   // then issue no attribute changes.
   static std::mutex mu;
   static size_t attr_smem[64][8] = {};
-  static int cached_per_sm[64][8][13][2] = {};
-  static size_t cached_smem[64][8][13][2] = {};
+  static int cached_per_sm[64][8][WARPS_168 + 1][2] = {};
+  static size_t cached_smem[64][8][WARPS_168 + 1][2] = {};
   int per_sm = 0;
   size_t smem = 0;
   {

@@ -54,9 +54,12 @@ typedef struct {
   double end_time_yr;   /* end_time (params.dat), used when d_t_end_yr is NULL       */
   long mxstep;          /* max internal steps per output interval (1e7, calculate_abundances.c:111) */
   int precision;        /* PDR_FP64 or PDR_MIXED                                      */
-  int warps_per_block;  /* warp integrator: warps (cells in flight) per block, 1..8; 0:
-                           8 (4 for register variants 2 and 3)                        */
-  int blocks_per_sm;    /* 0: as many as fit                                          */
+  int warps_per_block;  /* warp integrator: warps (cells in flight) per block, 1..8 (1..4
+                           for register variants 2 and 3); 0: 8, for variants 2 and 3 one
+                           block of the SM's 12 warps (4 for a network whose arrays do not
+                           fit that way, and where blocks_per_sm counts blocks)       */
+  int blocks_per_sm;    /* 0: as many as fit; n > 0: at most n (of 4 warps in register
+                           variants 2 and 3 unless warps_per_block says otherwise)    */
   int reg_variant;      /* warp integrator register budget (-1, the default: 1 for the
                            mixed form, 2 for FP64): 0 as needed (8 warps/SM),
                            1 at most 128 per thread (16 warps/SM, Nordsieck rows in
@@ -198,7 +201,9 @@ int pdr_chem_solve_batched_noalloc(const pdr_net *net, int ncell, double *d_abun
 /* Autotuner: times launch shapes (warps per block, register variant, refill
  * policy) on copies of the first ncell_sample cells of the given inputs (the
  * inputs are not modified; the best of two runs per shape) and writes the
- * fastest into opts, keeping its other fields.  Allocates temporary device
+ * fastest into opts, keeping its other fields (blocks_per_sm becomes 0).  The
+ * 12-warp blocks of register variant 2 (warps_per_block 0), the FP64 default,
+ * are among them where ncell_sample fills one on every SM.  Allocates temporary device
  * buffers; call it before stream capture. */
 int pdr_chem_autotune(const pdr_net *net, int ncell_sample, const double *d_abundance,
                       const double *d_rate, const double *d_density, pdr_chem_opts *opts,
