@@ -165,8 +165,6 @@ int build_coolant_tables(pdr_coolant *c) {
   t.temps = up(c, temps, rc);
   t.col = up(c, col, rc);
   t.dcol = up(c, dcol, rc);
-  t.A = up(c, h.A, rc);
-  t.B = up(c, h.B, rc);
   t.freq = up(c, h.freq, rc);
   t.weights = up(c, h.weights, rc);
   {
@@ -175,7 +173,6 @@ int build_coolant_tables(pdr_coolant *c) {
     t.rweights = up(c, rw, rc);
   }
   t.energies = up(c, h.energies, rc);
-  t.line_of_pair = up(c, lop, rc);
   std::vector<int> rp;
   for (int i = 0; i < n; i++)
     for (int j = 0; j < i; j++) {

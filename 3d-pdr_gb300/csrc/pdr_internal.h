@@ -77,7 +77,6 @@ struct WarpTables {
   int rhs_len = 0;     // RHS terms per lane (balanced chunks)
   int nparts = 0;      // partial-sum slots (slot nparts is a constant zero)
   int plist_len = 0;   // partial slots summed per species
-  int jac_len = 0;     // Jacobian terms per species (padded)
   int2 *rab = nullptr;        // [nreac] reactant slots (a, b)
   double *nh_mask = nullptr;  // [nreac] 1 if the rate constant is multiplied by n_H
   // RHS f_i = sum over terms of (nu kn_r) * operand: operands are the slot
@@ -90,6 +89,9 @@ struct WarpTables {
   int2 *rhs_t = nullptr;      // [rhs_len][lanes] (kn index | (partial slot written after the term + 1) << 16,
                               //  operand | sign of nu << 31)
   int2 *pairs = nullptr;      // [npairs] slots (a, b) of each reactant pair
+  // (The block integrator's kernel reads rab, rhs_t, pairs, plist, h_*, bnd_*; the
+  // warp integrator's reads the packed form of them that follows, and its plain
+  // ones serve the host check of the tables.)
   // The warp integrator's term tables in one packed block of `wtab_words` ints,
   // which a block copies to shared memory (offsets in ints; words: TermWord,
   // JacWord, PairWord above):
@@ -109,9 +111,6 @@ struct WarpTables {
   int *kext_ptr = nullptr;    // [nkext+1] extra rate constant e = sum over kext_rn[kext_ptr[e]..kext_ptr[e+1])
   int2 *kext_rn = nullptr;    //   of nu * kn_r, (reaction r, nu) in reaction order
   int *plist = nullptr;       // [plist_len][lanes] partial slots of species `lane`
-  int *jac_rab = nullptr;     // [jac_len][lanes] reaction | slot a << 16 | slot b << 24
-  double *jac_nu = nullptr;   // [jac_len][lanes]
-  float *jac_nu_f = nullptr;  // [jac_len][lanes]
   double *xe_coef = nullptr;  // [lanes] electron-sum coefficient per slot
   float *xe_coef_f = nullptr; // the same in FP32 (the mixed forms' Newton matrix)
   // term-parallel Jacobian assembly (block integrator): the (row, column)
@@ -145,8 +144,7 @@ struct WarpTables {
     int off_ba = 0, off_d = 0, total = 0;   // storage offsets / size, in elements
     int nnz_b = 0;                          // trailing rows' leaf-column entries
     int nlev = 0, nul = 0;
-    int *perm = nullptr;      // [N] unknown (elimination order) -> slot (species, neq = x_e)
-    int *iperm = nullptr;     // [N] slot -> unknown
+    int *iperm = nullptr;     // [N] slot (species, neq = x_e) -> unknown, in elimination order
     int *a_ptr = nullptr;     // [a+1] leaf row r: storage [a_ptr[r], a_ptr[r+1])
     unsigned short *a_col = nullptr;   // column (unknown) of each leaf-row entry, ascending
     int *a_diag = nullptr;    // [a] storage position of the diagonal
@@ -228,9 +226,8 @@ struct CoolantTables {
   double *temps = nullptr;     // [npart][ntemp]
   double *col = nullptr;       // [npart][ntemp][nlev*nlev]
   double *dcol = nullptr;      // [npart][ntemp][nlev*nlev] col[k+1] - col[k] (0 for the last)
-  double *A = nullptr, *B = nullptr, *freq = nullptr, *weights = nullptr, *rweights = nullptr;   // rweights: 1/weights
+  double *freq = nullptr, *weights = nullptr, *rweights = nullptr;   // rweights: 1/weights
   double *energies = nullptr;  // [nlev] level energies, erg
-  int *line_of_pair = nullptr; // [nlev*nlev] radiative line of (i,j), i>j, else -1
   int nrad = 0;
   int *rad_pairs = nullptr;    // [nrad] pairs i*nlev+j, i>j, with A or B nonzero either way
   double *pair_tmp2 = nullptr; // [nrad] 2 h nu^3 / c^2

@@ -690,21 +690,6 @@ int build_device_tables(pdr_net *net) {
     std::vector<int> pl(w.plist_len * G, slot /* zero slot */);
     for (int i = 0; i < G; i++)
       for (size_t k = 0; k < parts[i].size(); k++) pl[k * G + i] = parts[i][k];
-    // per-species Jacobian term lists
-    std::vector<std::vector<Term>> per(G);
-    for (auto &t : terms) per[t.i].push_back(t);
-    w.jac_len = 1;
-    for (auto &p : per) w.jac_len = std::max<int>(w.jac_len, (int)p.size());
-    std::vector<int> jr(w.jac_len * G, 0);   // reaction | a << 16 | b << 24
-    std::vector<double> jn(w.jac_len * G, 0.0);
-    std::vector<float> jnf(w.jac_len * G, 0.0f);
-    for (int i = 0; i < G; i++)
-      for (size_t k = 0; k < per[i].size(); k++) {
-        const int r = per[i][k].r;
-        jr[k * G + i] = r | (rab[r].x << 16) | (rab[r].y << 24);
-        jn[k * G + i] = per[i][k].nu;
-        jnf[k * G + i] = (float)per[i][k].nu;
-      }
     std::vector<double> xe(G, 0.0);
     for (int i = 0; i < neq; i++) xe[i] = h.xe[i];
     // term-parallel Jacobian tables (both integrators)
@@ -866,9 +851,6 @@ int build_device_tables(pdr_net *net) {
     w.kext_ptr = upload(net, kext_ptr, rc2);
     w.kext_rn = upload(net, kext_rn, rc2);
     w.plist = upload(net, pl, rc2);
-    w.jac_rab = upload(net, jr, rc2);
-    w.jac_nu = upload(net, jn, rc2);
-    w.jac_nu_f = upload(net, jnf, rc2);
     w.xe_coef = upload(net, xe, rc2);
     {
       std::vector<float> xef(xe.begin(), xe.end());
@@ -889,7 +871,6 @@ int build_device_tables(pdr_net *net) {
       d.nnz_b = (int)plan.b_col.size();
       d.nlev = (int)plan.lev_ptr.size() - 1;
       d.nul = (int)plan.ul_ptr.size() - 1;
-      d.perm = upload(net, plan.perm, rc2);
       d.iperm = upload(net, plan.iperm, rc2);
       d.a_ptr = upload(net, plan.a_ptr, rc2);
       d.a_col = upload(net, plan.a_col, rc2);
