@@ -3,7 +3,10 @@
 //  rounding  sqrt_rn rounds as the IEEE operation and rcp_near is within 0.5 + 2^-35 ulp,
 //            whatever the FP32 unit's start value (moved by up to 2 ulp) -- on random operands
 //            and on those whose results lie nearest to the midpoint of two doubles
-// Usage: fp64_check rounding; exit 0 when every check holds.
+//  tables    every row of fp64_tables.inc against its definition
+//  functions the errors stated in fp64_fast.cuh, over the ranges the kernels use and at
+//            their ends; "ulp" is 2^-52 of the result
+// Usage: fp64_check rounding|tables|functions; exit 0 when every check holds.
 #include "../../3d-pdr_gb300/csrc/fp64_fast.cuh"
 
 #include <quadmath.h>
@@ -89,9 +92,115 @@ static int check_rounding() {
   return bad != 0;
 }
 
+typedef __float128 Q;
+
+static int check_tables() {
+  int bad = 0;
+  auto expect = [&](const char *what, int j, bool ok) {
+    if (!ok && bad++ < 10) std::printf("%s, row %d\n", what, j);
+  };
+  for (int j = 0; j < 1024; j++) {
+    const Q v = exp2q((Q)j / 1024);
+    expect("2^(j/1024) rounded", j, kExp2Tab[j].t == (double)v);
+    // the row's relative error, to nine digits
+    const Q d = v / kExp2Tab[j].t - 1;
+    expect("its relative error", j, fabsq(kExp2Tab[j].d - d) <= 1e-8Q * fabsq(d) + 1e-30Q);
+  }
+  Q rmax = 0;
+  for (int j = 0; j < 512; j++) {
+    const LogRow &r = kLogTab[j];
+    const Q v = -1024 * log2q((Q)r.c), grid = (Q)r.hi * 4294967296.0Q;
+    expect("-1024 log2(c) rounded", j, r.full == (double)v);
+    expect("hi on the 2^-32 grid", j, grid == floorq(grid));
+    expect("hi + lo", j, fabsq((Q)r.hi + r.lo - v) <= 1e-17Q);
+    // m c - 1 over the row's mantissas
+    for (int k = 0; k < 2; k++) rmax = fmaxq(rmax, fabsq((1 + (Q)(j + k) / 512) * r.c - 1));
+    expect("c of twelve bits", j, r.c * 4096.0f == std::floor(r.c * 4096.0f));
+  }
+  std::printf("largest |m c - 1|: %.3g\n", (double)rmax);
+  expect("m c - 1", 0, rmax < 1.0Q / 400);
+  return bad != 0;
+}
+
+static int check_functions() {
+  const int N = 300000;
+  const double U = 2.220446049250313e-16;
+  int bad = 0;
+  auto expect = [&](const char *what, double worst, double bound) {
+    std::printf("%-12s %.4g (bound %.4g)\n", what, worst, bound);
+    if (!(worst <= bound)) bad++;
+  };
+  auto rel = [](double got, Q want) { return (double)fabsq(((Q)got - want) / want); };
+  double e = 0, l = 0, l1 = 0, p = 0, x2 = 0;
+  for (int i = 0; i < N; i++) {
+    const double x = i % 7 == 0 ? uniform(-1e-3, 1e-3) : (i & 1) ? uniform(-40, 5) : uniform(-690, 690);
+    e = std::fmax(e, rel(exp_fast(x), expq(x)) / U);
+    // the rates' T/300 and T, columns, optical depths; near 1 the logarithm's leading bits cancel
+    const double y = i % 5 == 0 ? 1 + uniform(-0.01, 0.01) : i % 11 == 0 ? std::ldexp(uniform(1, 2), i % 2000 - 1000)
+                                                                              : std::exp(uniform(-60, 60));
+    const Q lq = 1024 * log2q(y);
+    const Log2 L = log2k(y);
+    l = std::fmax(l, (double)fabsq((Q)L.h + L.l - lq));
+    // its use: log10 of columns, which the shielding clamps at 12 from below
+    const double n = std::exp(uniform(std::log(1e12), std::log(1e30)));
+    l1 = std::fmax(l1, rel(log2k1(n), 1024 * log2q(n)) / U);
+    const double b = uniform(-6, 6);
+    if (std::fabs(b * std::log2(y)) < 990) p = std::fmax(p, rel(powk(L, b), powq(y, b)) / U);
+    const int k = (int)(rng() % 1800000) - 900000;
+    const double r = uniform(-2, 2), a = uniform(1, 2);
+    x2 = std::fmax(x2, rel(exp2_times(a, k, r), a * exp2q(((Q)k + r) / 1024)) / U);
+  }
+  expect("exp_fast", e, 0.502);
+  expect("log2k", l, 1.5e-14);
+  expect("log2k1", l1, 1.0);   // the row's rounding and the sum's
+  expect("powk", p, 0.70);
+  // the roundings of a times the row and of the sum; at |r| = 2 the series' first term left
+  // out, (2 C1)^3/60 of 2 C1^2 (0.17), and the FP32 rounding of those kept (0.1)
+  expect("exp2_times", x2, 1.27);
+  for (double x : {0.0, -0.0}) expect("exp_fast(0)", std::fabs(exp_fast(x) - 1), 0);
+  expect("exp_fast(-800)", exp_fast(-800.0), 0);
+  // f2d and d2f: exact where they have to be, truncation elsewhere
+  double conv = 0;
+  for (int i = 0; i < N; i++) {
+    const float f = (float)(std::ldexp(uniform(1, 2), (int)(rng() % 252) - 126)) * (i & 1 ? 1.0f : -1.0f);
+    if (f2d(f) != (double)f || d2f((double)f) != f) conv++;
+    const double d = std::ldexp(uniform(1, 2), (int)(rng() % 240) - 120);
+    const float t = d2f(d);
+    if (!((double)t <= d && d < (double)std::nextafter(t, INFINITY))) conv++;
+  }
+  if (f2d(0.0f) != 0 || d2f(0.0) != 0 || d2f(1e-40) != 0 || d2f(-1e-300) != 0) conv++;
+  expect("f2d, d2f", conv, 0);
+  double rs = 0, dv = 0, any = 0;
+  for (g_seed_ulps = -1; g_seed_ulps <= 1; g_seed_ulps++)
+    for (int i = 0; i < N / 3; i++) {
+      const double w = std::ldexp(uniform(1, 4), 2 * ((int)(rng() % 60) - 30));
+      rs = std::fmax(rs, rel(rsqrt_fast(w), 1 / sqrtq(w)) / U);
+      const double a = std::ldexp(uniform(1, 2), (int)(rng() % 280) - 140) * (i & 1 ? 1 : -1);
+      double b = std::ldexp(uniform(1, 2), (int)(rng() % 280) - 140) * (i & 2 ? 1 : -1);
+      if (i % 9 == 0) b = 1 + std::ldexp((double)(i % 50), -52);
+      if (i % 13 == 0) b = 2 - std::ldexp((double)(1 + i % 50), -52);
+      const Q q = (Q)a / b;
+      const double got = div_fast(a, b);
+      dv = std::fmax(dv, (double)(fabsq(got - q) / std::ldexp(1.0, std::ilogb(a / b) - 52)));
+      const double c = std::ldexp(uniform(1, 2), (int)(rng() % 2040) - 1020), d = std::ldexp(uniform(1, 2), (int)(rng() % 2040) - 1020);
+      if (div_any(c, d) != c / d) any++;
+    }
+  expect("rsqrt_fast", rs, 0.64);
+  expect("div_fast", dv, 0.5 + std::ldexp(1.0, -35));
+  for (double c : {0.0, 1.0, -3.0, 5e-324, 1e308, (double)INFINITY})
+    for (double d : {0.0, 7.0, -2.0, 5e-324, 1e308, (double)INFINITY}) {
+      const double g = div_any(c, d), w = c / d;
+      if (__double_as_longlong(g) != __double_as_longlong(w) && !(std::isnan(g) && std::isnan(w))) any++;
+    }
+  expect("div_any", any, 0);
+  return bad != 0;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "rounding") return check_rounding();
-  std::printf("usage: fp64_check rounding\n");
+  if (what == "tables") return check_tables();
+  if (what == "functions") return check_functions();
+  std::printf("usage: fp64_check rounding|tables|functions\n");
   return 2;
 }

@@ -22,7 +22,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["rounding"])
+@pytest.mark.parametrize("what", ["rounding", "tables", "functions"])
 def test_functions(check, what):
     r = subprocess.run([check, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
