@@ -148,18 +148,23 @@ __device__ __forceinline__ Log2 log2k(double x) {
   L.l = fma(r * r, fma(r, c3, -0.5 * K_LN2), t) + f2d(bl);
   return L;
 }
-// the same to one double
-__device__ __forceinline__ double log2k1(double x) {
+// log10(x) to one double (0.545 ulp for x of 1e12 and more), x positive normal: the
+// row's exact part times log10(2)/1024 and the series, already in tens, in the
+// last sum alone
+__device__ __forceinline__ double log10_fast(double x) {
+  constexpr double LG = 0.00029397460514060664;   // log10(2)/1024, to 9e-18 of it
+  constexpr double M = 0.43429448190325182;       // 1/ln 10
   const int hx = hi32(x);
   const int e = (hx >> 20) - 1023;
   const LogRow *row = &kLogTab[(hx >> 11) & 511];
   const double m = __hiloint2double((hx & 0xfffff) | 0x3ff00000, lo32(x));
-  const double r = fma(m, f2d(__ldg(&row->c)), -1.0);
-  const double a = f2d((float)(e * 1024)) + __ldg(&row->full);
+  const float2 cl = __ldg(reinterpret_cast<const float2 *>(&row->c));
+  const double r = fma(m, f2d(cl.x), -1.0);
+  const double a = f2d((float)(e * 1024)) + __ldg(&row->hi);   // exact
   const float rf = d2f(r);
-  // (1024/ln 2) (1 - r/2 + r^2/3 - r^3/4)
-  const double c2 = add_rel(-0.5 * K_LN2, 1.4426950f, rf * fmaf(rf, fmaf(rf, -0.4f, 0.5f), -2.0f / 3.0f));
-  return fma(r, fma(r, c2, K_LN2), a);
+  // (1/ln 10) (1 - r/2 + r^2/3 - r^3/4)
+  const double c2 = add_rel(-0.5 * M, 1.7371779f, rf * fmaf(rf, fmaf(rf, -0.4f, 0.5f), -2.0f / 3.0f));
+  return fma(a, LG, fma(r, fma(r, c2, M), f2d(cl.y * (float)LG)));
 }
 // b L -> the integer k and remainder r of 1024 log2(x^b); returns k
 __device__ __forceinline__ int pow_arg(const Log2 &L, double b, double &r) {

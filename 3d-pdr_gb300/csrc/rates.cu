@@ -663,8 +663,7 @@ __global__ void __launch_bounds__(RATES_THREADS, 3) rates_kernel(const __grid_co
           if (S.has_hd) R.hd = s * h2shield_fast(nhd, S, A.ph.v_turb);
         }
         if (S.has_co) {
-          constexpr double LG = 0.00029397460514060664;   // log10(2)/1024
-          const double u = fp64::log2k1(nco + 1.0) * LG, w = fp64::log2k1(nh2 + 1.0) * LG;
+          const double u = fp64::log10_fast(nco + 1.0), w = fp64::log10_fast(nh2 + 1.0);
           const double tl = R.av2 * (xlambda_lbar(u, w, linear) * (1.0 / 1.086));
           bool jump;
           double s = scatter_fast(tl, jump);
