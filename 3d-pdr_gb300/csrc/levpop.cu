@@ -623,16 +623,13 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
       int *perm = reinterpret_cast<int *>(dinv + n4);
       // rows as columns of R^T would be: lane i scales rows i and i + 32
       float s0 = 1.0f, s1 = 1.0f;
-      bool fits = true;
+      int top = 0;   // the largest magnitude's upper word
       for (int i = lane; i < n4; i += 32) {
         float mx = 0.0f;
         for (int l = 0; l < n4; l++) {
-          float v = i == l ? 1.0f : 0.0f;
-          if (i < n && l < n) {
-            const double r = R[i * n + l];
-            v = fp64::d2f(r);
-            fits &= (fp64::hi32(r) & 0x7fffffff) < 0x47e00000;   // 2^127
-          }
+          const double r = (i < n && l < n) ? R[i * n + l] : (i == l ? 1.0 : 0.0);
+          const float v = fp64::d2f(r);
+          top = max(top, fp64::hi32(r) & 0x7fffffff);
           Mf[i * ld + l] = v;
           mx = fmaxf(mx, fabsf(v));
         }
@@ -642,7 +639,7 @@ __global__ void __launch_bounds__(256) levpop_kernel(const __grid_constant__ Coo
         else s1 = sc;
       }
       __syncwarp();
-      ok = __all_sync(FULL, fits);
+      ok = __all_sync(FULL, top < 0x47e00000);   // 2^127
       bool good = false;
       if (ok) {
         ok = lu_pp(Mf, n4, ld, upan, perm, dinv);
