@@ -219,8 +219,7 @@ __device__ __forceinline__ double div_any(double a, double b) {
   if (ea - 64u > 1918u || eb - 64u > 1918u || ea - eb + 959u > 1918u) return a / b;
   return div_fast(a, b);
 }
-// q, within 2^-35 ulp of the rounded result, or the neighbour that is nearer to
-// the exact one: res is the exact residual of q, whose magnitude passes `half`
+// q, within 1.4 ulp of the exact result, or the neighbour that is nearer to it: res is the exact residual of q, whose magnitude passes `half`
 // (the bits of a positive value) where the exact result lies half an ulp beyond
 // q.  Below a power of two the ulp is half as large.  Integer operations only.
 __device__ __forceinline__ double settle(double q, double res, long long half) {
@@ -228,18 +227,19 @@ __device__ __forceinline__ double settle(double q, double res, long long half) {
   const long long below = half - ((qb & 0xfffffffffffffll) ? 0ll : 1ll << 52);
   return __longlong_as_double(qb + (r >= 0 ? (mag > half ? 1 : 0) : (mag >= below ? -1 : 0)));
 }
-// sqrt(x), rounded: seven FP64 instructions where x is within FP32's normal range
-// (six leave out 2^-88 of the root; the exact residual x - g^2 settles the rest:
-// at the midpoint above g it is g ulp(g) + ulp(g)^2/4, in whole ulp(g)^2 beyond it)
+// sqrt(x), rounded: five FP64 instructions where x is within FP32's normal range.
+// From y near 1/sqrt(x), g = x y and r = (1 - x y^2)/2 < 2^-20, the root is
+// g (1 + r + 3 r^2/2 + ...), to 2^-62 and the rounding of g; the exact residual
+// x - g^2 settles it: at the midpoint above g it is g ulp(g) + ulp(g)^2/4, in whole
+// ulp(g)^2 beyond it.
 __device__ __forceinline__ double sqrt_rn(double x) {
   if ((unsigned)hi32(x) - 0x38200000u > 0x0f000000u) return __dsqrt_rn(x);   // zero, negative, tiny, huge, NaN
   const float y0 = rsqrt_approx(d2f(x));
-  const double y = f2d(y0), g = x * y, h = scale2(y, -1);
-  const double r = fma(-g, h, 0.5);              // (1 - x y^2)/2
-  const double g1 = fma(g, r, g), h1 = fma(h, r, h);
-  const double g2 = fma(fma(-g1, g1, x), h1, g1);
-  const long long eg = (long long)((unsigned)hi32(g2) >> 20) - 1023;
-  return settle(g2, fma(-g2, g2, x), __double_as_longlong(g2) + (eg - 52) * (1ll << 52));
+  const double y = f2d(y0), g = x * y;
+  const double r = fma(-g, scale2(y, -1), 0.5);
+  const double g1 = fma(g, fma(r, f2d(1.5f * d2f(r)), r), g);
+  const long long eg = (long long)((unsigned)hi32(g1) >> 20) - 1023;
+  return settle(g1, fma(-g1, g1, x), __double_as_longlong(g1) + (eg - 52) * (1ll << 52));
 }
 // 1/sqrt(x), x positive normal within FP32's range
 __device__ __forceinline__ double rsqrt_fast(double x) {
