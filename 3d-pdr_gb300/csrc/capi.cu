@@ -5,6 +5,7 @@
 // device arrays and a stream so a caller can keep state resident in HBM and
 // capture the calls in a CUDA graph.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -36,7 +37,7 @@ int launch_chem_warp(const pdr_net *net, int ncell, double *ab, const double *ra
 int launch_chem_cta(const pdr_net *net, int ncell, double *ab, const double *rate, const double *dens,
                     const double *tend, const pdr_chem_opts &o, int *status, int *stats, int *queue,
                     int *fb_list, int *fb_count, const int *cell_list, const int *total_ptr, bool mixed,
-                    int grid, void *scratch, cudaStream_t st, const int *sm_limit = nullptr, int grid_sms = 1);
+                    int grid, void *scratch, cudaStream_t st, const int *sm_limit, int grid_sms, bool shares);
 size_t chem_cta_global_bytes(const pdr_net *net, bool mixed, int grid);
 size_t chem_cta_smem(const pdr_net *net, bool mixed, bool *mat_smem);
 int chem_cta_blocks_per_sm(const pdr_net *net, bool mixed);
@@ -102,6 +103,7 @@ struct Scratch {
   void *cta = nullptr;       // block integrator: per-block rate constants (and matrices)
   size_t cta_bytes = 0;
   int *sm_limit = nullptr;   // solver instances: SMs their running launch may keep (null: all)
+  std::atomic<bool> limited{false};   // solver instances: pdr_solver_limit_sms has been called
 };
 static std::mutex g_mu;
 static Scratch g_scratch[64];
@@ -225,6 +227,8 @@ static int solve_core(const pdr_net *net, int ncell, double *ab, const double *r
       return PDR_E_ARG;
     }
   }
+  // the launch shares the GPU: it was given a number of SMs, or its instance has been limited before
+  const bool shares = o.max_sms > 0 || s->limited.load(std::memory_order_relaxed);
   const int grid_main = one_per_cell ? ncell : cta_grid(net, o, mixed, sms);
   size_t bytes = std::max(cta_bytes_needed(net, o, sms), chem_cta_global_bytes(net, mixed, grid_main));
   if (grow) {
@@ -235,11 +239,11 @@ static int solve_core(const pdr_net *net, int ncell, double *ab, const double *r
     return PDR_E_ARG;
   }
   rc = launch_chem_cta(net, ncell, ab, rate, dens, tend, o, status, stats, s->counters + 0, s->redo, s->counters + 2,
-                       nullptr, nullptr, mixed, grid_main, s->cta, st, s->sm_limit, eff_sms(o, sms));
+                       nullptr, nullptr, mixed, grid_main, s->cta, st, s->sm_limit, eff_sms(o, sms), shares);
   if (rc || !mixed) return rc;
   return launch_chem_cta(net, ncell, ab, rate, dens, tend, o, status, stats, s->counters + 1, nullptr, nullptr,
                          s->redo, s->counters + 2, false, cta_grid(net, o, false, sms), s->cta, st, s->sm_limit,
-                         eff_sms(o, sms));
+                         eff_sms(o, sms), shares);
 }
 
 }  // namespace pdr
@@ -421,6 +425,7 @@ int pdr_solver_limit_sms(pdr_solver *v, int max_sms, void *control_stream) {
     set_error("pdr_solver_limit_sms: invalid argument");
     return PDR_E_ARG;
   }
+  v->s.limited.store(true, std::memory_order_relaxed);
   v->h_words[1] = max_sms;
   cudaError_t e = cudaMemcpyAsync(v->s.sm_limit, v->h_words + 1, sizeof(int), cudaMemcpyHostToDevice,
                                   (cudaStream_t)control_stream);

@@ -1362,7 +1362,7 @@ int chem_cta_blocks_per_sm(const pdr_net *net, bool mixed) {
 int launch_chem_cta(const pdr_net *net, int ncell, double *ab, const double *rate, const double *dens,
                     const double *tend, const pdr_chem_opts &o, int *status, int *stats, int *queue,
                     int *fb_list, int *fb_count, const int *cell_list, const int *total_ptr, bool mixed,
-                    int grid, void *scratch, cudaStream_t st, const int *sm_limit, int grid_sms) {
+                    int grid, void *scratch, cudaStream_t st, const int *sm_limit, int grid_sms, bool shares) {
   const WarpTables &T = net->cta;
   if (!net->cta_ok || T.lanes > 256) return PDR_E_NET;
   CtaArgs A;
@@ -1400,8 +1400,24 @@ int launch_chem_cta(const pdr_net *net, int ncell, double *ab, const double *rat
   auto k = cta_kernel(variant);
   cudaError_t ea = ensure_smem_attr(variant, smem);
   if (ea != cudaSuccess) return cuda_fail(ea, "cudaFuncSetAttribute(chem_cta_kernel)");
-  k<<<grid, T.lanes, smem, st>>>(A, ncell, total_ptr, ms ? 1 : 0);
-  cudaError_t e = cudaGetLastError();
+  // A launch that shares its SMs with others asks for all of their memory as
+  // shared memory.  Left to the driver, two blocks of the full network (195.9 KiB)
+  // get the 196 KiB split, which an SM keeps until it is empty: the reduced
+  // network's blocks did not fit beside one that stayed, and the 80/20 served
+  // stream's p50 was 104 ms in place of 44, its p99 20.4 s in place of 15.5.  A
+  // launch that has the GPU to itself keeps the larger L1 (900 cells 374 ms, 381
+  // with the whole memory shared).
+  cudaLaunchAttribute carve{};
+  carve.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  carve.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)T.lanes);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &carve;
+  cfg.numAttrs = shares ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, A, ncell, total_ptr, ms ? 1 : 0);
   return e == cudaSuccess ? 0 : cuda_fail(e, "chem_cta_kernel launch");
 }
 

@@ -73,7 +73,8 @@ typedef struct {
   int integrator;       /* 0: automatic (one warp per cell for 32 ODE species, else
                            one block per cell), 1: warp per cell, 2: block per cell */
   int max_sms;          /* 0: the persistent grid spans every SM; n > 0: only n SMs'
-                           worth of blocks, leaving the rest to concurrent solves */
+                           worth of blocks, leaving the rest to concurrent solves, and an
+                           SM's memory split so that their blocks fit beside its own */
 } pdr_chem_opts;
 
 void pdr_chem_opts_default(pdr_chem_opts *opts);
@@ -123,7 +124,9 @@ int pdr_solver_set_max_sms(pdr_solver *solver, int max_sms);
  * is written by a 4-byte copy on control_stream, which must not be the run's
  * own stream (the copy would wait for the run).  Each pdr_solver_run starts
  * again with every SM of its grid.  Results do not depend on the allowance.
- * Work-queue mode (refill 0) only; no counterpart in the reference. */
+ * Work-queue mode (refill 0) only; no counterpart in the reference.  The runs of
+ * an instance after its first limit (or with max_sms set, as the server's) leave
+ * the SMs' memory split so that other launches' blocks fit beside their own. */
 int pdr_solver_limit_sms(pdr_solver *solver, int max_sms, void *control_stream);
 void pdr_solver_free(pdr_solver *solver);
 
