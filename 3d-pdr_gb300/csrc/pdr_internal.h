@@ -71,12 +71,17 @@ struct PairWord {
 // CTA-per-cell integrator (lanes = 32*ceil(neq/32), at least 64; neq <= 252
 // so that a slot fits the 8-bit field of the packed term tables).
 // Slot convention: 0..neq-1 species, neq = electron (x_e), neq+1 = constant 1.
+// The struct is a kernel parameter, and the offsets of its fields change what the
+// compiler makes of the warp kernel: without pad_a..pad_c 64 cells take 21.5 to 22.1
+// ms in place of 21.1 to 21.3 (means of six runs on three machines), and 21.6 and
+// 21.8 with two other orders of the fields.  Larger batches do not notice.
 struct WarpTables {
   int neq = 0, nreac = 0;
   int lanes = 0;       // table stride: threads of the group
   int rhs_len = 0;     // RHS terms per lane (balanced chunks)
   int nparts = 0;      // partial-sum slots (slot nparts is a constant zero)
   int plist_len = 0;   // partial slots summed per species
+  int pad_a = 0;
   int2 *rab = nullptr;        // [nreac] reactant slots (a, b)
   double *nh_mask = nullptr;  // [nreac] 1 if the rate constant is multiplied by n_H
   // RHS f_i = sum over terms of (nu kn_r) * operand: operands are the slot
@@ -111,6 +116,7 @@ struct WarpTables {
   int *kext_ptr = nullptr;    // [nkext+1] extra rate constant e = sum over kext_rn[kext_ptr[e]..kext_ptr[e+1])
   int2 *kext_rn = nullptr;    //   of nu * kn_r, (reaction r, nu) in reaction order
   int *plist = nullptr;       // [plist_len][lanes] partial slots of species `lane`
+  void *pad_b[3] = {};
   double *xe_coef = nullptr;  // [lanes] electron-sum coefficient per slot
   float *xe_coef_f = nullptr; // the same in FP32 (the mixed forms' Newton matrix)
   // term-parallel Jacobian assembly (block integrator): the (row, column)
@@ -144,6 +150,7 @@ struct WarpTables {
     int off_ba = 0, off_d = 0, total = 0;   // storage offsets / size, in elements
     int nnz_b = 0;                          // trailing rows' leaf-column entries
     int nlev = 0, nul = 0;
+    void *pad_c = nullptr;
     int *iperm = nullptr;     // [N] slot (species, neq = x_e) -> unknown, in elimination order
     int *a_ptr = nullptr;     // [a+1] leaf row r: storage [a_ptr[r], a_ptr[r+1])
     unsigned short *a_col = nullptr;   // column (unknown) of each leaf-row entry, ascending
