@@ -698,9 +698,10 @@ template <> struct RegVariant<3> { static constexpr int threads = 384, min_block
 // instruction cache, then the FP64 pipe.  So the hot code is kept small -- one
 // call site for the RHS, the setup and the solve, rolled loops, divisions side
 // by side -- and the FP64 instructions few (about 75 a step in the mixed form).
-// 64,000 cells, mixed: 684 -> 500 ms; 5,003: 71.3 -> 50.4 ms; 64 (one warp per
-// block busy, latency alone): 28.9 -> 22.0 ms; 1,500 cells in FP64 through host
-// buffers: 80.3 -> 71.5 ms.  Results are bit-identical.
+// 64,000 cells, mixed: 684 -> 495 ms; 5,003: 71.3 -> 49.5 ms; 64 (latency, several
+// of the cells on one SM, as the warps take them from one counter): 28.3 -> 21.1 ms;
+// 1,500 cells in FP64 through host buffers: 80.9 -> 71.2 ms.  Results are the same
+// bits, but for FP64 pivot reciprocals that may round the other way once in 2^35.
 template <int NSP, bool MIXED, int RV>
 __global__ void __launch_bounds__(RegVariant<RV>::threads, RegVariant<RV>::min_blocks)
     chem_warp_kernel(const __grid_constant__ ChemArgs A, int total_cells, const int *total_ptr) {

@@ -592,7 +592,7 @@ constexpr int RATES_THREADS = 256;
 // lanes are kept full -- items of every phase are flattened over the batch's
 // cells -- and the powers and exponentials take 3 to 9 FP64 instructions each
 // (fp64_fast.cuh) instead of 19 (exp) and 95 (pow).  100,003 cells of the
-// reduced network take 1.26 ms (one warp per cell with the library functions:
+// reduced network take 1.25 ms (one warp per cell with the library functions:
 // 24.2 ms), 8,000 of the full one 0.46 ms (8.13 ms).  Against 113-bit values
 // a (T/300)^b is 6.7e-17 off (rms, as with a correctly rounded pow) and
 // a exp(-g/T) 6.7e-17 (1.3e-15 where g/T is rounded first).
